@@ -123,9 +123,9 @@ ctb_status ctb_set_filter_mode(ctb_ctx* ctx, int mode);
  * thread; 3 = 16x16, 1 per thread; all with 32 angles per staged chunk; and
  * the 32x32 tile with 16 (4) and 64 (5) angles per chunk, which sum every
  * voxel's angles in the same order as shape 0 and so give its result bit for
- * bit. Without tuning a job gets a shape from its size alone (32x32 once its
- * tiles x slice groups reach the SM count, 32x16 above a quarter of it, else
- * 16x16). With the autotuner
+ * bit. (A chunk is half the ring of staged windows, one window per angle and
+ * group of four slices.) Without tuning a job gets a shape from its size alone:
+ * 32x32, or 32x16 or 16x16 where its tiles would leave SMs idle. With the autotuner
  * on, the first job of each size bucket {ceil(n / 64), ceil(angles / 180),
  * floor(log2(ceil(depth / 4)))} times every shape on its own data (that call
  * synchronises) and the fastest is kept for the bucket; batches use a tuned

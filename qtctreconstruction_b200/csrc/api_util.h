@@ -72,8 +72,8 @@ struct Guard {
     explicit Guard(ctb_ctx* c) : ctx(c), lock(c->mu) { cudaSetDevice(c->device); }
 };
 
-// Device angle table (double2 cs[na] then float2 csf[na]) filled from host
-// degrees; synchronous on the context's stream.
+// Device angle table (trig_bytes(na)) filled from host degrees; synchronous on
+// the context's stream.
 ctb_status fill_trig(ctb_ctx* ctx, const float* angles_deg, int na, void* table);
 // Cached uniform table or the context's explicit-list table.
 ctb_status trig_table(ctb_ctx* ctx, const float* angles_deg, int na, Trig* out);

@@ -10,20 +10,47 @@
 // reconstruction, denormalised with the slice's span and minimum (span folded
 // into the filter output, minimum added in the epilogue).
 //
-// Work decomposition: a work item is a TX x TY voxel tile of four slices (the
-// float4 lanes of the filtered rows) of one job. Per angle, the detector window
-// that the tile can touch (WIN bins) is staged into shared memory by the
-// bulk-copy engine (cp.async.bulk, completion on an mbarrier), CA angles per
-// chunk, double-buffered. The tile origin's detector coordinate is evaluated in
-// double precision once per angle and split into the window start and a
-// fractional offset, so each thread evaluates u in float on small numbers
-// (|u_local| < WIN): the interpolation position is ~10x more accurate than the
-// reference's float u of magnitude ~sq. Each of the 256 threads accumulates
-// VPT voxels x 4 slices in registers; voxels outside the circle load nothing.
-// Six shapes are compiled: four tile shapes with 32-angle chunks (32x32 / 4
-// per thread, the default; 64x32 / 8; 32x16 / 2; 16x16 / 1) and the 32x32 tile
-// with 16- and 64-angle chunks; bp_default_variant picks one of the first four
-// from the job's size, the context's autotuner times all six per size bucket.
+// Work decomposition: a work item is a TX x TY voxel tile of one or two groups of
+// four slices (the float4 lanes of the filtered rows) of one job. Per angle, the
+// detector window that the tile can touch (WIN bins) is staged into shared memory
+// by the bulk-copy engine (cp.async.bulk), in a ring of stages; the warps take
+// turns as the producer and meet only through the stages' mbarriers. The tile
+// origin's detector coordinate is evaluated in double precision once per angle
+// and split into the window start and a fractional offset, so each thread
+// evaluates u in float on small numbers (|u_local| < WIN): the interpolation
+// position is ~10x more accurate than the reference's float u of magnitude ~sq.
+// Six shapes are compiled: four tile shapes (32x32, the default; 64x32; 32x16;
+// 16x16) and the 32x32 tile with half and twice the ring; bp_default_variant
+// picks among 32x32, 32x16 and 16x16 from the job's size, the context's autotuner
+// times all six per size bucket.
+//
+// What bounds it and why this split: interpolating each voxel on its own reads
+// two 16-byte taps per voxel and angle, and such a kernel ran at 0.92 of the
+// shared-memory load bandwidth (18.28 ms at 512^3 x 720). Neighbouring voxels
+// share taps along the axis where u changes slowly (coefficient at most
+// sqrt(1/2) bins per voxel), so a thread owns columns of four voxels along that
+// slow axis and its lanes run along the other (fast) one: a column's taps are 3,
+// 4 or 5 consecutive bins (3.6 on average over the angles, against 8), read
+// once, and lanes next to each other read bins next to each other, without bank
+// conflicts. Each voxel adds three taps with hat weights; which three depends on
+// the slow coefficient alone (four patterns, column_taps), and two slice groups
+// share the weights. The kernel is then bound by issue: 48 packed FP32x2
+// operations of two issue cycles and about 62 other instructions per column and
+// angle of 8 slices (11.03 ms at 512^3 x 720; FMA pipe 67 %, shared memory 75 %
+// busy; with two of the taps read only, 10.95 ms). Measured and not kept: tap
+// differences with saturating weights, which share the first tap's sum within a
+// column (11.72 ms), one slice group per item (13.4 ms) or four (11.07 ms), 64 or
+// 128 registers (12.4 and 11.3 ms against 80).
+//
+// The slow axis is x for angles with |sin| > |cos| and y for the others, so a
+// tile runs through the angles in the order of the table (Trig): first those
+// with columns along x, then, after the accumulators changed places through
+// shared memory, those with columns along y; within each, the angles whose slow
+// coefficient is positive, then (columns walked from the other end) negative,
+// and within those one tap pattern after the other. Small tiles split the angles
+// of a stage over SPLIT groups of threads, whose sums are added in a fixed order
+// at the end, so that a thread always has columns to share taps in and its
+// serial chain of angles is short.
 //
 // One kernel serves both shapes of work: a single job with one CTA per item,
 // or a batch of jobs (BpBatch) on a persistent grid that takes items from an
@@ -31,36 +58,49 @@
 // so a job's output is bit-identical alone and in any mix of the same shape.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "ctb_internal.h"
 
 namespace ctb {
 namespace {
 
-constexpr int NBUF = 2;       // chunk buffers
 constexpr int THREADS = 256;
 constexpr float kRound = 12582912.0f;   // 1.5 * 2^23: x + kRound rounds x to an integer
 constexpr int kRoundBits = 0x4B400000;  // bit pattern of kRound
 
-// A tile shape: TX x TY voxels of four slices, VPT voxels per thread along x
-// (spaced XS = TX / VPT apart), CA angles per staged chunk and WIN bins per
-// staged window (>= ceil(sqrt((TX-1)^2 + (TY-1)^2)) + 3 plus rounding margin:
-// the taps of every tile position lie in [ws, ws + span + 3)). MINB is the
-// launch-bounds occupancy target (registers 65536 / (256 MINB)).
-template <int TX_, int TY_, int VPT_, int CA_, int WIN_, int MINB_>
+// A tile shape: TX x TY voxels in columns of V, a ring of NST stages of CA / 2
+// windows (one per angle and slice group) and WIN bins per window: with a span of
+// sqrt((TX-1)^2 + (TY-1)^2) bins, the taps of every column lie in bins 0 ..
+// floor(span + 2) + 2 of the window. MINB is the launch-bounds occupancy target (registers 65536 / (256 MINB)).
+constexpr int V = 4;
+template <int TX_, int TY_, int CA_, int WIN_, int NST_, int MINB_, bool PAIR_>
 struct Shape {
-    static constexpr int TX = TX_, TY = TY_, VPT = VPT_, CA = CA_, WIN = WIN_, MINB = MINB_;
-    static constexpr int XS = TX / VPT;
-    static_assert(XS * TY == THREADS, "256 threads per CTA");
-    static_assert(CA <= THREADS, "one thread per staged angle");
+    static constexpr int TX = TX_, TY = TY_, CA = CA_, WIN = WIN_, MINB = MINB_;
+    static constexpr bool PAIR = PAIR_;
+    // Stages, and how many the producer works ahead: it refills the slot of two
+    // stages back, so a warp may lag one stage without holding it up (refilling
+    // the last stage's slot made every producer wait for the slowest warp: 13.3
+    // against 11.4 ms at 512^3 x 720).
+    static constexpr int NST = NST_, AHEAD = NST - 2;
+    static constexpr int SW = CA / 2;                                // windows per stage
+    static constexpr int COLS = TX * TY / V;                         // columns of a tile
+    static constexpr int SPLIT = COLS >= THREADS ? 1 : THREADS / COLS;  // groups that share a chunk's angles
+    static constexpr int GT = THREADS / SPLIT;                       // threads per group
+    static constexpr int NC = COLS / GT;                             // columns per thread
+    static_assert(NC * GT == COLS && GT * SPLIT == THREADS, "whole columns per thread");
+    static_assert(TX % 16 == 0 && TY % 16 == 0 && GT % TX == 0 && GT % TY == 0, "lanes along either axis");
+    static_assert(GT % 32 == 0, "a warp is in one group");
+    static_assert(SW <= 32 && SW % (2 * SPLIT) == 0, "a lane per staged angle, whole turns of the groups");
     static_assert(WIN <= kBpWindowMax, "window within the filtered-row guard");
+    static_assert(SPLIT * V * GT <= SPLIT * TX * TY, "the exchange buffer holds every group's sums");
 };
-using V0 = Shape<32, 32, 4, 32, 52, 4>;  // the general-purpose shape
-using V1 = Shape<64, 32, 8, 32, 76, 2>;  // wide tiles: half the staging per voxel
-using V2 = Shape<32, 16, 2, 32, 40, 4>;  // half-height tiles: twice the CTAs
-using V3 = Shape<16, 16, 1, 32, 28, 4>;  // small tiles for small slices
-using V4 = Shape<32, 32, 4, 16, 52, 4>;  // the general shape with 16-angle chunks (half the staging buffer)
-using V5 = Shape<32, 32, 4, 64, 52, 2>;  // the general shape with 64-angle chunks (half the chunk barriers)
+using V0 = Shape<32, 32, 32, 48, 5, 3, true>;  // the general-purpose shape
+using V1 = Shape<64, 32, 32, 76, 4, 2, false>;  // wide tiles: less staging per voxel
+using V2 = Shape<32, 16, 32, 40, 5, 3, true>;  // half-height tiles: twice the CTAs
+using V3 = Shape<16, 16, 32, 28, 5, 3, true>;  // small tiles for small slices
+using V4 = Shape<32, 32, 16, 48, 5, 3, true>;  // the general shape with half the ring
+using V5 = Shape<32, 32, 64, 48, 4, 2, true>;  // the general shape with twice the ring (half the stages)
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
     return static_cast<unsigned>(__cvta_generic_to_shared(p));
@@ -76,6 +116,9 @@ __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned
                  "r"(bytes)
                  : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes,
                                           unsigned long long* bar) {
     asm volatile(
@@ -83,6 +126,13 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
             smem_u32(dst)),
         "l"(src), "r"(bytes), "r"(smem_u32(bar))
         : "memory");
+}
+// 16 bytes from a 32-bit shared address (volatile: stays between the barriers
+// around it).
+__device__ __forceinline__ float4 lds128(unsigned a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
 }
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
     unsigned ok;
@@ -107,6 +157,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsig
     if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
     for (unsigned it = 0; it < (1u << 22); ++it) {
+        __nanosleep(32);  // leave the issue slots to the warps that work
         if (mbar_try_wait(bar, parity)) return true;
         if (global_ns() - t0 > limit_ns) break;
     }
@@ -134,46 +185,94 @@ __global__ void k_wait_selftest(unsigned limit_us, unsigned* err) {
 // The fields the inner loop reads every angle come first: one 16-byte
 // shared-memory broadcast per warp and angle.
 struct AngleRec {
-    float f0;  // tile-origin u minus window start
-    float c, s;
+    float f0;      // u of the tile corner with the lowest slow term, minus the window start
+    float cf, as;  // u per voxel along the fast axis; |u per voxel| along the slow axis
     int edge;      // the window reaches a detector edge: decide taps like the reference
-    int ws;        // window start bin (unguarded coordinates)
-    float cf, sf;  // the reference's float cos/sin (edge decisions only)
-    int pad;
+    float rc, rs;  // the reference's float cos/sin (edge decisions only)
+    int pad[2];
 };
 
 template <class C>
 struct BpSmem {
-    float4 win[NBUF][C::CA][C::WIN];
-    AngleRec rec[NBUF][C::CA];
-    unsigned long long bar[NBUF];
+    static constexpr int NST = C::NST;
+    float4 win[NST][C::SW][C::WIN];
+    float2 ex[C::SPLIT * C::TX * C::TY];     // exchange of accumulators between threads
+    AngleRec rec[NST][C::SW + C::SPLIT];     // a record is read ahead of its use
+    unsigned long long full[NST], empty[NST];
+    int meta[NST];                           // stage: angles | group << 8 | some angle has `edge` set << 16
+    int first[kBpGroups];                    // first stage of each group of the angle order
+    int start[kBpGroups + 1];                // first angle of each group; na
+    int total;                               // stages of the item
+    int dead;                                // a wait gave up
 };
 
-// Backproject one tile (x0, y0) of slice group zg of job J. `chunks` counts
-// the chunks this CTA has consumed so far (mbarrier phases continue across
-// items). Returns false when a bounded wait gave up (block-uniform).
-template <class C>
-__device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, int x0, int y0, unsigned& chunks,
+// One column of V = 4 voxels at one angle. w: shared address of the window bin of the column's
+// lowest voxel, f1 its fraction minus 1, as <= sqrt(1/2) (to rounding) the step
+// in u. Voxel v lies frac + v as bins above w, in interval m_v or m_v + 1, where
+// m_v = floor(v as) depends on the pattern P alone (the range of as):
+//   P = 0: as in [0, 1/3):   m = 0 0 0 0, taps 0..2      P = 2: [1/2, 2/3): m = 0 0 1 1, taps 0..3
+//   P = 1: as in [1/3, 1/2): m = 0 0 0 1, taps 0..3      P = 3: [2/3, ..]:  m = 0 0 1 2, taps 0..4
+// so with y = frac + v as - m_v - 1 in [-1, 1] its value is max(-y, 0) w[m_v] +
+// (1 - |y|) w[m_v + 1] + max(y, 0) w[m_v + 2] (two taps for v = 0): 11 packed
+// FP32x2 operations per pair of slices and column and 3 to 5 shared loads, where
+// a tap pair per voxel takes 8 of each. ZG groups of four slices share the
+// weights; group p's window lies p WIN bins on.
+template <int P, int ZG, int WIN>
+__device__ __forceinline__ void column_taps(unsigned w, float f1, float as,
+                                            float2 (&acc)[V][2 * ZG]) {
+    constexpr int T = P == 0 ? 3 : P == 3 ? 5 : 4;
+    constexpr int m0[V] = {0, 0, P >= 2 ? 1 : 0, P == 0 ? 0 : P == 3 ? 2 : 1};
+    float c[V][3];
+    c[0][0] = -f1;
+    c[0][1] = 1.0f + f1;
+    c[0][2] = 0.0f;
+#pragma unroll
+    for (int v = 1; v < V; ++v) {
+        const float y = fmaf(static_cast<float>(v), as, f1 - static_cast<float>(m0[v]));
+        c[v][0] = fmaxf(-y, 0.0f);
+        c[v][1] = 1.0f - fabsf(y);
+        c[v][2] = fmaxf(y, 0.0f);
+    }
+#pragma unroll
+    for (int m = 0; m < T; ++m) {
+        float2 q[2 * ZG];
+#pragma unroll
+        for (int p = 0; p < ZG; ++p) {
+            const float4 r = lds128(w + static_cast<unsigned>((p * WIN + m) * sizeof(float4)));
+            q[2 * p] = make_float2(r.x, r.y);
+            q[2 * p + 1] = make_float2(r.z, r.w);
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            if (m < m0[v] || m > m0[v] + (v == 0 ? 1 : 2)) continue;
+            const float2 W = make_float2(c[v][m - m0[v]], c[v][m - m0[v]]);
+#pragma unroll
+            for (int h = 0; h < 2 * ZG; ++h) acc[v][h] = __ffma2_rn(W, q[h], acc[v][h]);
+        }
+    }
+}
+
+// Backproject one tile (x0, y0) of ZG slice groups from zg on of job J. `stages`
+// counts the stages this CTA has consumed so far (mbarrier phases continue
+// across items). Returns false when a bounded wait gave up (block-uniform).
+template <class C, int ZG>
+__device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, int x0, int y0, unsigned& stages,
                                         unsigned* err) {
-    constexpr int TX = C::TX, TY = C::TY, VPT = C::VPT, XS = C::XS, CA = C::CA, WIN = C::WIN;
+    constexpr int TX = C::TX, TY = C::TY, WIN = C::WIN, NC = C::NC;
+    constexpr int SA = C::SW / ZG;           // angles per stage
+    constexpr int NST = C::NST, AHEAD = C::AHEAD;
+    constexpr int NS = 4 * ZG, NH = 2 * ZG;  // slices, pairs of slices
     const int t = threadIdx.x;
-    const int lx = t % XS, ly = t / XS;
     const int n = J.n, nz = J.nz, na = J.na, sq = J.sq;
     const double ctr = J.ctr;  // voxel-grid centre (the mask radius too)
     const float radf = static_cast<float>(ctr);
 
-    float add[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int z = 4 * zg + j;
-        float a = 0.0f;
-        if (J.stats && J.denorm != CTB_DENORM_NONE && z < nz) {
-            const float4 st = J.stats[z];
-            // CUDABackend.cu:676-681 adds the minimum only when max > min
-            a = (J.denorm == CTB_DENORM_CUDA && !(st.y - st.x > 0.0f)) ? 0.0f : st.x;
-        }
-        add[j] = a;
-    }
+    auto offset = [&](int z) {  // the slice's minimum (0 in normalised units)
+        if (!J.stats || J.denorm == CTB_DENORM_NONE || z >= nz) return 0.0f;
+        const float4 st = J.stats[z];
+        // CUDABackend.cu:676-681 adds the minimum only when max > min
+        return (J.denorm == CTB_DENORM_CUDA && !(st.y - st.x > 0.0f)) ? 0.0f : st.x;
+    };
 
     // Tiles entirely outside the reconstruction circle hold only the offset.
     {
@@ -181,153 +280,333 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
         const double dx = fmax(0.0, fmax(x0 - ctr, ctr - xe));
         const double dy = fmax(0.0, fmax(y0 - ctr, ctr - ye));
         if (dx * dx + dy * dy > ctr * ctr) {
-            const int y = y0 + ly;
-#pragma unroll
-            for (int k = 0; k < VPT; ++k) {
-                const int x = x0 + lx + XS * k;
-                if (x >= n || y >= n) continue;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int z = 4 * zg + j;
-                    if (z < nz) J.out[(static_cast<long long>(z) * n + y) * n + x] = add[j];
+            for (int z = 4 * zg; z < min(nz, 4 * zg + NS); ++z) {
+                const float o = offset(z);
+                for (int i = t; i < TX * TY; i += THREADS) {
+                    const int x = x0 + i % TX, y = y0 + i / TX;
+                    if (x < n && y < n) J.out[(static_cast<long long>(z) * n + y) * n + x] = o;
                 }
             }
             return true;
         }
     }
 
-    const double dcd = J.dc;
-    const float dcf = static_cast<float>(J.dc);
-    const double ox = static_cast<double>(x0) - ctr, oy = static_cast<double>(y0) - ctr;
-    const float4* plane = J.filt + static_cast<long long>(zg) * na * J.pitch;
-    const int nch = (na + CA - 1) / CA;
+    // A stage is up to SA angles of one group of the angle order (Trig), so
+    // its tap pattern is the same for all. Warp 0 lists the groups' first stages.
+    const int warp = t / 32, lane = t & 31;
+    if (warp == 0) {
+        const int begin = lane > 0 && lane <= kBpGroups ? J.trig.end[lane - 1] : 0;
+        const int count = lane < kBpGroups ? J.trig.end[lane] - begin : 0;
+        int sum = (count + SA - 1) / SA;
+        const int own = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int q = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += q;
+        }
+        if (lane < kBpGroups) {
+            S.first[lane] = sum - own;
+            S.start[lane] = begin;
+        }
+        if (lane == 31) {
+            S.total = sum;
+            S.start[kBpGroups] = na;
+        }
+    }
+    __syncthreads();
+    const int total = S.total;
 
-    auto issue = [&](int c, int b) {
-        const int a0 = c * CA;
-        const int cnt = min(CA, na - a0);
-        if (t < cnt) {
-            const int a = a0 + t;
+    // One warp fills the item's stage i (the CTA's stage s).
+    // Its slot was last used NST stages ago: every warp arrived on `empty` after
+    // reading it.
+    auto produce = [&](unsigned s, int i) {
+        const int slot = s % NST;
+        const unsigned use = s / NST;
+        bool ok = *static_cast<volatile int*>(&S.dead) == 0;
+        if (ok && use > 0 && !mbar_wait_bounded(&S.empty[slot], (use - 1) & 1, err)) ok = false;
+        ok = __all_sync(0xffffffffu, ok);
+        // the last group that starts at or before stage i
+        const int grp = __popc(__ballot_sync(0xffffffffu, lane < kBpGroups && S.first[lane & (kBpGroups - 1)] <= i)) - 1;
+        const int pos = S.start[grp] + (i - S.first[grp]) * SA;
+        const int cnt = min(SA, S.start[grp + 1] - pos);
+        const bool along = grp < kBpGroups / 2, flip = (grp / 4) & 1;
+        if (!ok) {  // nothing is copied any more; the consumers' waits still end
+            if (lane == 0) {
+                *static_cast<volatile int*>(&S.dead) = 1;
+                S.meta[slot] = SA;
+                mbar_expect_tx(&S.full[slot], 0);
+            }
+            return;
+        }
+        int a = 0, ws = 0, edge = 0;
+        if (lane < cnt) {
+            a = J.trig.order[pos + lane];
             const double2 tc = J.trig.cs[a];
             const float2 tf = J.trig.csf[a];
-            const double uo = ox * tc.x - oy * tc.y + dcd;
+            const double uo = (x0 - ctr) * tc.x - (y0 - ctr) * tc.y + J.dc;
             const double umin = uo + fmin(0.0, (TX - 1) * tc.x) + fmin(0.0, -(TY - 1) * tc.y);
             const double umax = uo + fmax(0.0, (TX - 1) * tc.x) + fmax(0.0, -(TY - 1) * tc.y);
-            const int ws = static_cast<int>(floor(umin)) - 1;
+            ws = static_cast<int>(floor(umin)) - 1;
+            // u = uo + x cos - y sin over the tile's voxels (x, y): columns
+            // along x or along y, walked from the end where the slow term is
+            // lowest
+            const double fast = along ? -tc.y : tc.x, slow = along ? tc.x : -tc.y;
             AngleRec r;
-            r.f0 = static_cast<float>(uo - ws);
-            r.c = static_cast<float>(tc.x);
-            r.s = static_cast<float>(tc.y);
-            r.ws = ws;
-            r.cf = tf.x;
-            r.sf = tf.y;
+            r.f0 = static_cast<float>(uo + (flip ? ((along ? TX : TY) - 1) * slow : 0.0) - ws);
+            r.cf = static_cast<float>(fast);
+            r.as = static_cast<float>(flip ? -slow : slow);
             // taps near bin 0 or bin sq-1: the reference's float u decides them
             // (the CUDA backend's per-tap bounds need no rule: bins outside
             // [0, sq) are zeros of the guard)
-            r.edge = (J.edge_rule && (umin < 2.0 || umax > sq - 3.0)) ? 1 : 0;
-            r.pad = 0;
-            S.rec[b][t] = r;
-            bulk_load(&S.win[b][t][0], plane + static_cast<long long>(a) * J.pitch + J.guard + ws,
-                      WIN * sizeof(float4), &S.bar[b]);
+            edge = J.edge_rule && (umin < 2.0 || umax > sq - 3.0);
+            r.edge = edge;
+            r.rc = tf.x;
+            r.rs = tf.y;
+            r.pad[0] = r.pad[1] = 0;
+            S.rec[slot][lane] = r;
         }
-        if (t == 0) mbar_expect_tx(&S.bar[b], static_cast<unsigned>(cnt * WIN * sizeof(float4)));
+        edge = __any_sync(0xffffffffu, edge);
+        if (lane == 0) S.meta[slot] = cnt | grp << 8 | (edge ? 1 << 16 : 0);
+        __syncwarp();
+        // the arrival publishes the records; the copies complete the stage
+        if (lane == 0) mbar_expect_tx(&S.full[slot], static_cast<unsigned>(cnt * ZG * WIN * sizeof(float4)));
+        __syncwarp();
+        if (lane < cnt) {
+            const float4* row = J.filt + (static_cast<long long>(zg) * na + a) * J.pitch + J.guard + ws;
+#pragma unroll
+            for (int p = 0; p < ZG; ++p)
+                bulk_load(&S.win[slot][lane * ZG + p][0], row + static_cast<long long>(p) * na * J.pitch,
+                          WIN * sizeof(float4), &S.full[slot]);
+        }
     };
 
-    float4 acc[VPT];
+    // this thread's columns: group g takes the angles g, g + SPLIT, ... of a
+    // stage; column k has fast coordinate `fast` and slow coordinates 4 col(k)
+    // .. 4 col(k) + 3 (counted from the other end of the tile when flipped)
+    const int g = t / C::GT, tg = t % C::GT;
+    float2 acc[NC][V][NH];
 #pragma unroll
-    for (int k = 0; k < VPT; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float fx = static_cast<float>(lx), fy = static_cast<float>(ly);
-    // positions inside the reconstruction circle (SerialBackend.cpp:220-224);
-    // the others are written as the offset only, so their taps are never loaded
-    unsigned inside_mask = 0;
-    {
-        const float yy = static_cast<float>(y0 + ly) - radf;
+    for (int k = 0; k < NC; ++k)
 #pragma unroll
-        for (int k = 0; k < VPT; ++k) {
-            const float xx = static_cast<float>(x0 + lx + XS * k) - radf;
-            if (!(xx * xx + yy * yy > radf * radf)) inside_mask |= 1u << k;
+        for (int v = 0; v < V; ++v)
+#pragma unroll
+            for (int h = 0; h < NH; ++h) acc[k][v][h] = make_float2(0.f, 0.f);
+    bool along_x = S.start[kBpGroups / 2] > 0, flipped = false;
+    int fast = 0, col[NC];
+    bool live[NC];  // some voxel of the column inside the circle
+    auto inside = [&](int x, int y) {  // SerialBackend.cpp:220-224
+        const float xx = static_cast<float>(x) - radf, yy = static_cast<float>(y) - radf;
+        return !(xx * xx + yy * yy > radf * radf);
+    };
+    auto map_columns = [&] {
+        const int F = along_x ? TY : TX;
+        fast = tg % F;
+#pragma unroll
+        for (int k = 0; k < NC; ++k) {
+            col[k] = tg / F + (C::GT / F) * k;
+            live[k] = false;
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const int s = V * col[k] + v;
+                live[k] |= along_x ? inside(x0 + s, y0 + fast) : inside(x0 + fast, y0 + s);
+            }
         }
-    }
-
-    // all buffers are idle between items: chunk g of this CTA uses buffer g & 1
-    issue(0, chunks & 1);
-    __syncthreads();
-    for (int c = 0; c < nch; ++c) {
-        const unsigned g = chunks + c;
-        const int b = g & 1;
-        if (c + 1 < nch) issue(c + 1, (g + 1) & 1);
-        // A failed wait leaves stale window data; the block then stops as a
-        // whole at the barrier below (the decision is block-uniform).
-        const bool landed = mbar_wait_bounded(&S.bar[b], (g >> 1) & 1, err);
-        const int cnt = min(CA, na - c * CA);
-        for (int j = 0; j < cnt; ++j) {
-            const AngleRec r = S.rec[b][j];
-            const float4* w = S.win[b][j];
-            const float ub = fmaf(fx, r.c, fmaf(-fy, r.s, r.f0));
-            const float c8 = static_cast<float>(XS) * r.c;
-            if (!r.edge) {
-                // i = floor(u) by rounding u - 1/2 with the kRound addition (no
-                // conversion-unit instructions); at an exact tie u = i + 1 the taps
-                // shift to (i, i+1) with weights (0, 1), the same value
-                const float ubh = ub - 0.5f;
+    };
+    auto flip_columns = [&] {  // the columns' voxels in the other order
+        flipped = !flipped;
+        const int ncol = (along_x ? TX : TY) / V;
 #pragma unroll
-                for (int k = 0; k < VPT; ++k) {
-                    if (!(inside_mask & (1u << k))) continue;
-                    const float uh = fmaf(static_cast<float>(k), c8, ubh);
-                    const float tr = uh + kRound;
-                    const int i = __float_as_int(tr) - kRoundBits;
-                    const float d = uh - (tr - kRound);  // frac(u) - 1/2
-                    const float w1 = d + 0.5f;
-                    const float w0 = 0.5f - d;
-                    const float4 lo = w[i], hi = w[i + 1];
-                    acc[k].x = fmaf(w1, hi.x, fmaf(w0, lo.x, acc[k].x));
-                    acc[k].y = fmaf(w1, hi.y, fmaf(w0, lo.y, acc[k].y));
-                    acc[k].z = fmaf(w1, hi.z, fmaf(w0, lo.z, acc[k].z));
-                    acc[k].w = fmaf(w1, hi.w, fmaf(w0, lo.w, acc[k].w));
+        for (int k = 0; k < NC; ++k) {
+            col[k] = ncol - 1 - col[k];
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+                float2 q = acc[k][0][h];
+                acc[k][0][h] = acc[k][3][h];
+                acc[k][3][h] = q;
+                q = acc[k][1][h];
+                acc[k][1][h] = acc[k][2][h];
+                acc[k][2][h] = q;
+            }
+        }
+    };
+    // Hand the sums of columns along x to the threads of the columns along y,
+    // two slices at a time. Voxel (x, y) of group g sits at y TX + (x ^ y mod
+    // 16): distinct banks for 16 lanes in x or in y.
+    auto exchange = [&] {
+        if (flipped) flip_columns();
+        float2* buf = S.ex + g * TX * TY;
+        const int yf = fast;
+        int xs[NC];
+#pragma unroll
+        for (int k = 0; k < NC; ++k) xs[k] = V * col[k];
+        along_x = false;
+        map_columns();
+#pragma unroll
+        for (int h = 0; h < NH; ++h) {
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < NC; ++k)
+#pragma unroll
+                for (int v = 0; v < V; ++v) buf[yf * TX + ((xs[k] + v) ^ (yf & 15))] = acc[k][v][h];
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < NC; ++k)
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    const int y = V * col[k] + v;
+                    acc[k][v][h] = buf[y * TX + (fast ^ (y & 15))];
                 }
-            } else {
+        }
+    };
+    map_columns();
+
+    // The warps take turns as the producer and meet only through the stages'
+    // barriers.
+    if (warp < min(AHEAD, total)) produce(stages + warp, warp);
+    bool landed = true;
+    for (int i = 0; i < total; ++i, ++stages) {
+        const int slot = stages % NST;
+        if (warp == i % (THREADS / 32) && i + AHEAD < total) produce(stages + AHEAD, i + AHEAD);
+        // A failed wait leaves stale window data; the block then stops as a
+        // whole at the end of the item (the decision is block-uniform).
+        if (!mbar_wait_bounded(&S.full[slot], (stages / NST) & 1, err)) {
+            landed = false;
+            *static_cast<volatile int*>(&S.dead) = 1;
+        }
+        const int meta = S.meta[slot], cnt = meta & 0xff, grp = (meta >> 8) & 0xff;
+        if (along_x && grp >= kBpGroups / 2) exchange();
+        if (flipped != (((grp / 4) & 1) != 0)) flip_columns();
+        const float fi = static_cast<float>(fast);
+        float fj[NC];
+        bool some = false;
+#pragma unroll
+        for (int k = 0; k < NC; ++k) {
+            fj[k] = static_cast<float>(V * col[k]);
+            some |= live[k];
+        }
+        if (some && landed && g < cnt) {
+            // 32-bit shared addresses of this group's first record and window;
+            // the window's is offset so that adding 16 times the bits of
+            // floor(u) + kRound gives the tap's
+            unsigned ra = smem_u32(&S.rec[slot][g]);
+            unsigned wa = smem_u32(&S.win[slot][g * ZG][0]) - (static_cast<unsigned>(kRoundBits) << 4);
+            auto run = [&](auto pattern) {
+                constexpr int P = decltype(pattern)::value;
+                float4 rec = lds128(ra);
+                const unsigned end = wa + static_cast<unsigned>((cnt - g + C::SPLIT - 1) / C::SPLIT) * (C::SPLIT * ZG * WIN * 16u);
+                while (wa != end) {
+                    const float rf0 = rec.x, rcf = rec.y, ras = rec.z;
+                    ra += C::SPLIT * sizeof(AngleRec);
+                    rec = lds128(ra);  // the next angle's
+#pragma unroll
+                    for (int k = 0; k < NC; ++k) {
+                        if (NC > 1 && !live[k]) continue;
+                        const float u = fmaf(fi, rcf, fmaf(fj[k], ras, rf0));
+                        const float tr = __fadd_rd(u, kRound);  // floor(u), no conversion-unit instruction
+                        column_taps<P, ZG, WIN>(wa + (__float_as_uint(tr) << 4), u - (tr - (kRound - 1.0f)), ras,
+                                                acc[k]);
+                    }
+                    wa += C::SPLIT * ZG * WIN * sizeof(float4);
+                }
+            };
+            if (meta >> 16) {
                 // SerialBackend.cpp:229-239 evaluates u = (xx cos - yy sin) + dc in
                 // float without fused multiply-add and keeps the tap pair only when
                 // 0 <= floor(u) and floor(u) + 1 < sq; that decision is reproduced
                 // here exactly, the interpolation itself uses the accurate u.
+                const float dcf = static_cast<float>(J.dc);
+                for (int j = g; j < cnt; j += C::SPLIT) {
+                    const AngleRec r = S.rec[slot][j];
+                    const float4* w = S.win[slot][j * ZG];
 #pragma unroll
-                for (int k = 0; k < VPT; ++k) {
-                    if (!(inside_mask & (1u << k))) continue;
-                    const float u = fmaf(static_cast<float>(k), c8, ub);
-                    const float fl = floorf(u);
-                    const int i = static_cast<int>(fl);
-                    const float xs = static_cast<float>(x0 + lx + XS * k) - radf;
-                    const float ys = static_cast<float>(y0 + ly) - radf;
-                    const float us = __fadd_rn(__fsub_rn(__fmul_rn(xs, r.cf), __fmul_rn(ys, r.sf)), dcf);
-                    const int is = static_cast<int>(floorf(us));
-                    const bool ok = (is >= 0) && (is + 1 < sq);
-                    const float w1 = ok ? u - fl : 0.0f;
-                    const float w0 = ok ? 1.0f - (u - fl) : 0.0f;
-                    const float4 lo = w[i], hi = w[i + 1];
-                    acc[k].x = fmaf(w1, hi.x, fmaf(w0, lo.x, acc[k].x));
-                    acc[k].y = fmaf(w1, hi.y, fmaf(w0, lo.y, acc[k].y));
-                    acc[k].z = fmaf(w1, hi.z, fmaf(w0, lo.z, acc[k].z));
-                    acc[k].w = fmaf(w1, hi.w, fmaf(w0, lo.w, acc[k].w));
+                    for (int k = 0; k < NC; ++k) {
+#pragma unroll
+                        for (int v = 0; v < V; ++v) {
+                            const float uv = fmaf(static_cast<float>(v), r.as, fmaf(fi, r.cf, fmaf(fj[k], r.as, r.f0)));
+                            const float fl = floorf(uv);
+                            const int iv = static_cast<int>(fl);
+                            const int sl = V * col[k] + v;
+                            const int sa = flipped ? (along_x ? TX : TY) - 1 - sl : sl;
+                            const float xs = static_cast<float>(x0 + (along_x ? sa : fast)) - radf;
+                            const float ys = static_cast<float>(y0 + (along_x ? fast : sa)) - radf;
+                            const float us = __fadd_rn(__fsub_rn(__fmul_rn(xs, r.rc), __fmul_rn(ys, r.rs)), dcf);
+                            const int is = static_cast<int>(floorf(us));
+                            const bool ok = !r.edge || ((is >= 0) && (is + 1 < sq));
+                            const float w1 = ok ? uv - fl : 0.0f;
+                            const float w0 = ok ? 1.0f - (uv - fl) : 0.0f;
+                            const float2 W0 = make_float2(w0, w0), W1 = make_float2(w1, w1);
+#pragma unroll
+                            for (int p = 0; p < ZG; ++p) {
+                                const float4 lo = w[p * WIN + iv], hi = w[p * WIN + iv + 1];
+                                float2(&A)[NH] = acc[k][v];
+                                A[2 * p] = __ffma2_rn(W1, make_float2(hi.x, hi.y),
+                                                      __ffma2_rn(W0, make_float2(lo.x, lo.y), A[2 * p]));
+                                A[2 * p + 1] = __ffma2_rn(W1, make_float2(hi.z, hi.w),
+                                                          __ffma2_rn(W0, make_float2(lo.z, lo.w), A[2 * p + 1]));
+                            }
+                        }
+                    }
                 }
+            } else {
+                const int pat = grp % 4;
+                if (pat == 0) run(std::integral_constant<int, 0>());
+                else if (pat == 1) run(std::integral_constant<int, 1>());
+                else if (pat == 2) run(std::integral_constant<int, 2>());
+                else run(std::integral_constant<int, 3>());
             }
         }
-        if (!__syncthreads_and(landed)) return false;
+        __syncwarp();
+        if ((t & 31) == 0) mbar_arrive(&S.empty[slot]);
     }
-    chunks += nch;
-
-    const int y = y0 + ly;
+    if (!__syncthreads_and(landed)) return false;
+    if (along_x) exchange();
+    if (flipped) flip_columns();
+    if constexpr (C::SPLIT > 1) {
+        // add the groups' sums in group order
+        static_assert(NC == 1, "one column per thread of a group");
 #pragma unroll
-    for (int k = 0; k < VPT; ++k) {
-        const int x = x0 + lx + XS * k;
-        if (x >= n || y >= n) continue;
-        const bool inside = inside_mask & (1u << k);
-        const float v[4] = {acc[k].x, acc[k].y, acc[k].z, acc[k].w};
+        for (int h = 0; h < NH; ++h) {
+            __syncthreads();
+            if (g > 0)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int z = 4 * zg + j;
-            if (z < nz) J.out[(static_cast<long long>(z) * n + y) * n + x] = (inside ? v[j] : 0.0f) + add[j];
+                for (int v = 0; v < V; ++v) S.ex[((g - 1) * V + v) * C::GT + tg] = acc[0][v][h];
+            __syncthreads();
+            if (g == 0)
+#pragma unroll
+                for (int s = 0; s < C::SPLIT - 1; ++s)
+#pragma unroll
+                    for (int v = 0; v < V; ++v) acc[0][v][h] = __fadd2_rn(acc[0][v][h], S.ex[(s * V + v) * C::GT + tg]);
         }
+        if (g > 0) return true;
+    }
+    const int x = x0 + fast;
+#pragma unroll
+    for (int j = 0; j < NS; ++j) {
+        const int z = 4 * zg + j;
+        if (z >= nz) break;
+        const float o = offset(z);
+#pragma unroll
+        for (int k = 0; k < NC; ++k)
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const int y = y0 + V * col[k] + v;
+                if (x >= n || y >= n) continue;
+                const float r = j & 1 ? acc[k][v][j / 2].y : acc[k][v][j / 2].x;
+                J.out[(static_cast<long long>(z) * n + y) * n + x] = (inside(x, y) ? r : 0.0f) + o;
+            }
     }
     return true;
+}
+
+// One item: the tile (x0, y0) of slice groups zg J.zgs ... of job J (a pair, or
+// one group where a pair would pass the last slice).
+template <class C>
+__device__ __forceinline__ bool bp_item(BpSmem<C>& S, const BpJob& J, int zi, int x0, int y0, unsigned& stages,
+                                        unsigned* err) {
+    const int zg = zi * J.zgs;
+    if constexpr (C::PAIR)
+        if (J.zgs == 2 && 4 * (zg + 1) < J.nz) return bp_tile<C, 2>(S, J, zg, x0, y0, stages, err);
+    return bp_tile<C, 1>(S, J, zg, x0, y0, stages, err);
 }
 
 // MODE 0: one job, one CTA per item (job 0 indexed statically keeps its fields
@@ -342,16 +621,20 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
     BpSmem<C>& S = *reinterpret_cast<BpSmem<C>*>(smem_raw);
     __shared__ int s_item;
     if (threadIdx.x == 0) {
-        for (int b = 0; b < NBUF; ++b) mbar_init(&S.bar[b], 1);
+        for (int b = 0; b < C::NST; ++b) {
+            mbar_init(&S.full[b], 1);
+            mbar_init(&S.empty[b], THREADS / 32);
+        }
+        S.dead = 0;
         mbar_fence_init();
     }
-    unsigned chunks = 0;
+    unsigned stages = 0;
     if constexpr (MODE == 0) {
         __syncthreads();
         const BpJob& J = batch.job[0];
         const int zg = blockIdx.x / J.tiles;
         const int tl = blockIdx.x - zg * J.tiles;
-        bp_tile<C>(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, chunks, err);
+        bp_item<C>(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, stages, err);
     } else if constexpr (MODE == 1) {
         __syncthreads();
         const int item = blockIdx.x;
@@ -361,7 +644,7 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
         const int local = item - static_cast<int>(J.first);
         const int zg = local / J.tiles;
         const int tl = local - zg * J.tiles;
-        bp_tile<C>(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, chunks, err);
+        bp_item<C>(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, stages, err);
     } else {
         for (;;) {
             if (threadIdx.x == 0) s_item = static_cast<int>(atomicAdd(counter, 1u));
@@ -374,7 +657,7 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
             const int local = item - static_cast<int>(J.first);
             const int zg = local / J.tiles;
             const int tl = local - zg * J.tiles;
-            if (!bp_tile<C>(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, chunks, err)) break;
+            if (!bp_item<C>(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, stages, err)) break;
             __syncthreads();  // shared state of this item is dead before the next item's staging
         }
     }
@@ -420,7 +703,7 @@ cudaError_t launch_many(const BpBatch& b, bool persistent, unsigned* d_counter, 
 
 template <class C>
 BpShape shape_of() {
-    return BpShape{C::TX, C::TY, C::VPT, C::CA, C::WIN};
+    return BpShape{C::TX, C::TY, C::TX * C::TY / THREADS, C::CA, C::WIN};
 }
 
 }  // namespace
@@ -441,16 +724,90 @@ BpShape bp_shape(int variant) {
     }
 }
 
+namespace {
+
+// Tiles of a shape that meet the reconstruction circle (the others are
+// filled without a loop over the angles).
+long long active_tiles(int n, const BpShape& sh, double ctr) {
+    long long count = 0;
+    for (int y0 = 0; y0 < n; y0 += sh.ty) {
+        const int ye = std::min(y0 + sh.ty, n) - 1;
+        const double dy = std::max(0.0, std::max(y0 - ctr, ctr - ye));
+        if (dy > ctr) continue;
+        const double half = std::sqrt(ctr * ctr - dy * dy);  // the circle's columns in these rows
+        const int lo = std::max(0, static_cast<int>(std::ceil(ctr - half)));
+        const int hi = std::min(n - 1, static_cast<int>(std::floor(ctr + half)));
+        if (hi >= lo) count += hi / sh.tx - lo / sh.tx + 1;
+    }
+    return count;
+}
+
+// Relative time of a launch with `items` work items on `sms` SMs: the items of
+// an SM times an item's cost. Three items fit an SM at once: up to that count
+// the fullest SM decides, a lone item taking 1.4 times its share of a full SM
+// (its 8 warps do not fill it); beyond it the SMs even out to half an item.
+// Costs per item (one or
+// two slice groups) relative to a 32x32 tile of one group, from the
+// backprojector's time at 512^2 x 64 x 720: 32x32 1.658 and 1.462 ms, 32x16
+// 1.822 and 1.640 ms, 16x16 2.173 and 2.082 ms.
+double launch_cost(int variant, int zgs, long long items, int sms) {
+    const double pair = variant == 2 ? 0.99 : variant == 3 ? 0.63 : 1.76;
+    const double one = variant == 2 ? 0.55 : variant == 3 ? 0.33 : 1.0;
+    const double per_sm = static_cast<double>(items) / sms;
+    const double rounds = per_sm <= 1.0 ? 1.4 : per_sm <= 3.0 ? std::ceil(per_sm) : per_sm + 0.5;
+    return (zgs == 2 ? pair : one) * rounds;
+}
+
+// Items of a job that run the angle loop, with zgs slice groups per item.
+long long active_items(const BpJob& J, int variant, int zgs) {
+    return active_tiles(J.n, bp_shape(variant), J.ctr) * (((J.nz + 3) / 4 + zgs - 1) / zgs);
+}
+
+}  // namespace
+
 int bp_default_variant(int n_out, int nz, int sms) {
-    // Measured on B200 (fbp of random sinograms, shapes forced): the 32x32
-    // tile is fastest once its CTAs reach the SM count (n >= 128 at 64
-    // slices); below that smaller tiles win by filling more SMs (n = 64,
-    // 16 slices: 16x16 0.025 ms, 32x16 0.031 ms, 32x32 0.044 ms). The 64x32
-    // tile never won and is left to the autotuner.
-    const long long ctas = static_cast<long long>((n_out + 31) / 32) * ((n_out + 31) / 32) * ((nz + 3) / 4);
-    if (ctas >= sms) return 0;
-    if (4 * ctas >= sms) return 2;
-    return 3;
+    // The shape whose launch is estimated fastest for the job alone; a smaller
+    // tile has to gain 15 % in the estimate, which leaves its own start-up cost
+    // out. Measured on B200, us, 32x32 / 32x16 / 16x16: 24.0 for 16x16
+    // at 64^2 x 16 x 101 (30.2 for 32x32); 40.4 / 38.3 / 50.6 at 128^2 x 32 x
+    // 201; 187.8 / 144.7 / 157.1 at 387^2 x 8 x 580; 1462 / 1640 / 2082 at 512^2
+    // x 64 x 720. The 64x32 tile and the other chunk sizes are left to the
+    // autotuner.
+    BpJob J;
+    J.n = n_out;
+    J.nz = nz;
+    J.ctr = static_cast<double>(n_out / 2);
+    int best = 0;
+    double least = 0.0;
+    for (const int v : {0, 2, 3}) {
+        const double t = std::min(launch_cost(v, 1, active_items(J, v, 1), sms),
+                                  launch_cost(v, 2, active_items(J, v, 2), sms));
+        if (v == 0 || t < 0.85 * least) {
+            best = v;
+            least = t;
+        }
+    }
+    return best;
+}
+
+void bp_number_items(BpBatch& b, int variant, int sms) {
+    // Pairs of slice groups share every weight (1.46 against 1.66 ms at 512^2 x
+    // 64 x 720) but make half as many items, which costs more than it gives
+    // where the items do not fill the SMs (58.8 against 40.4 us at 128^2 x 32
+    // x 201). A slice's result does not depend on the choice.
+    long long one = 0, two = 0;
+    for (int k = 0; k < b.njobs; ++k) {
+        one += active_items(b.job[k], variant, 1);
+        two += active_items(b.job[k], variant, 2);
+    }
+    const bool pair = variant != 1 && launch_cost(variant, 2, two, sms) < launch_cost(variant, 1, one, sms);
+    b.total = 0;
+    for (int k = 0; k < b.njobs; ++k) {
+        BpJob& J = b.job[k];
+        J.zgs = pair ? 2 : 1;
+        J.first = b.total;
+        b.total += static_cast<long long>(J.tiles) * (((J.nz + 3) / 4 + J.zgs - 1) / J.zgs);
+    }
 }
 
 FiltLayout filt_layout(int sq, int n_out) {
@@ -499,6 +856,7 @@ BpJob make_bp_job(const float4* d_filt, int nz, int na, const FiltLayout& fl, in
     J.tiles_x = (n_out + sh.tx - 1) / sh.tx;
     J.tiles = J.tiles_x * ((n_out + sh.ty - 1) / sh.ty);
     J.first = 0;
+    J.zgs = 1;
     return J;
 }
 
@@ -522,7 +880,10 @@ cudaError_t launch_backproject(const float4* d_filt, int nz, int na, const FiltL
     BpBatch b;
     b.njobs = 1;
     b.job[0] = make_bp_job(d_filt, nz, na, fl, n_out, trig, d_stats, denorm, d_out, variant, convention);
-    b.total = static_cast<long long>(b.job[0].tiles) * ((nz + 3) / 4);
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    bp_number_items(b, variant, sms);
     if (b.total > 0x7fffffffLL) return cudaErrorInvalidValue;
     switch (variant) {
     case 1: return launch_one<V1>(b, d_err, st);

@@ -100,7 +100,7 @@ ctb_status build(ctb_batch* b) {
         q.g = pad_geometry(j.bins);
         q.fl = filt_layout(q.g.sq, j.output_size);
         q.trig_off = off;
-        off += align_up((sizeof(double2) + sizeof(float2)) * static_cast<size_t>(j.num_angles));
+        off += align_up(trig_bytes(j.num_angles));
         q.filt_off = off;
         off += align_up(sizeof(float4) * static_cast<size_t>((j.depth + 3) / 4) * j.num_angles *
                         q.fl.pitch);
@@ -124,9 +124,7 @@ ctb_status build(ctb_batch* b) {
             const std::vector<float> uni = uniform_angles(j.num_angles);
             CTB_TRY(fill_trig(ctx, uni.data(), j.num_angles, table));
         }
-        Trig trig;
-        trig.cs = static_cast<const double2*>(table);
-        trig.csf = reinterpret_cast<const float2*>(static_cast<const double2*>(table) + j.num_angles);
+        const Trig trig = trig_view(table, j.num_angles);
         const float2* d_Hc = nullptr;
         const float2* d_tw = nullptr;
         CTB_TRY(filter_tables(ctx, q.g, j.filter, &d_Hc, &d_tw));
@@ -174,12 +172,10 @@ ctb_status build(ctb_batch* b) {
         BpBatch p;
         const int v = var[by_na[k]];
         while (k < n && p.njobs < cap && var[by_na[k]] == v) {
-            BpJob J = bj[by_na[k]];
-            J.first = p.total;
-            p.total += static_cast<long long>(J.tiles) * ((J.nz + 3) / 4);
-            p.job[p.njobs++] = J;
+            p.job[p.njobs++] = bj[by_na[k]];
             ++k;
         }
+        bp_number_items(p, v, ctx->sms);
         b->bp.push_back(p);
         b->bp_variant.push_back(v);
     }

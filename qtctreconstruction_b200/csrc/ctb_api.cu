@@ -46,10 +46,6 @@ using namespace ctb;
 
 namespace ctb {
 
-// Fill a device angle table: na double2 (device sincospi) followed by na
-// float2 holding the reference's float cos/sin of degToRad(deg)
-// (SerialBackend.cpp:92-95, 198-204; Utils.cpp:44-46), computed here on the
-// host with the same libm calls.
 // A table upload from pageable host memory, complete on return. A plain
 // cudaMemcpy from pageable memory may return before its DMA has landed and is
 // ordered only against the legacy default stream, while the kernels run on
@@ -61,6 +57,10 @@ ctb_status upload(ctb_ctx* ctx, void* dst, const void* src, size_t bytes) {
     return CTB_OK;
 }
 
+// Fill a device angle table: na double2 (device sincospi) followed by na
+// float2 holding the reference's float cos/sin of degToRad(deg)
+// (SerialBackend.cpp:92-95, 198-204; Utils.cpp:44-46), computed here on the
+// host with the same libm calls, then the backprojector's angle order.
 ctb_status fill_trig(ctb_ctx* ctx, const float* angles_deg, int na, void* table) {
     std::vector<float2> csf(na);
     for (int a = 0; a < na; ++a) {
@@ -72,7 +72,7 @@ ctb_status fill_trig(ctb_ctx* ctx, const float* angles_deg, int na, void* table)
     CTB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // previous users of the buffers are done
     CTB_TRY(upload(ctx, d_deg, angles_deg, sizeof(float) * na));
     CTB_TRY(upload(ctx, static_cast<double2*>(table) + na, csf.data(), sizeof(float2) * na));
-    CTB_LAUNCH(ctx, launch_trig(d_deg, na, static_cast<double2*>(table), ctx->stream));
+    CTB_LAUNCH(ctx, launch_trig(d_deg, na, trig_view(table, na), ctx->stream));
     CTB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return CTB_OK;
 }
@@ -81,7 +81,7 @@ ctb_status fill_trig(ctb_ctx* ctx, const float* angles_deg, int na, void* table)
 // in float) are cached per count; an explicit angle list is re-uploaded only
 // when it differs from the previous one.
 ctb_status trig_table(ctb_ctx* ctx, const float* angles_deg, int na, Trig* out) {
-    const size_t bytes = (sizeof(double2) + sizeof(float2)) * na;
+    const size_t bytes = trig_bytes(na);
     void* table = nullptr;
     if (!angles_deg) {
         auto it = ctx->trig_uniform.find(na);
@@ -105,8 +105,7 @@ ctb_status trig_table(ctb_ctx* ctx, const float* angles_deg, int na, Trig* out) 
             ++ctx->user_angles_gen;
         }
     }
-    out->cs = static_cast<const double2*>(table);
-    out->csf = reinterpret_cast<const float2*>(static_cast<const double2*>(table) + na);
+    *out = trig_view(table, na);
     return CTB_OK;
 }
 

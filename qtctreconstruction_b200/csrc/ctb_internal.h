@@ -75,14 +75,41 @@ struct DevBuf {
 //   csf: the reference's own float (cos, sin) of degToRad(deg) (Utils.cpp:44-46
 //        with libm cosf/sinf), used only to reproduce its discontinuous
 //        decisions (which taps exist at the detector edges) bit for bit.
+//   order, end: the angles in the order the backprojector takes them, in groups
+//        g = 4 s + p that end at end[g] (the last at na). s: the angles whose
+//        detector coordinate u = x cos - y sin changes least along x (|sin| >
+//        |cos|) with cos >= 0 (s = 0), with cos < 0 (1), the others with sin <=
+//        0 (2) and with sin > 0 (3). p: the smaller coefficient's magnitude in
+//        [0, 1/3), [1/3, 1/2), [1/2, 2/3), [2/3, 1), the ranges that share a tap
+//        pattern. Angles keep their given order in a group.
+constexpr int kBpGroups = 16;
 struct Trig {
     const double2* cs = nullptr;
     const float2* csf = nullptr;
+    const uint16_t* order = nullptr;
+    const int* end = nullptr;  // kBpGroups
 };
+
+// One angle table: double2 cs[na], float2 csf[na] (trig_base_bytes), then the
+// backprojector's order: int end[kBpGroups], uint16_t order[na] (order_bytes).
+inline size_t trig_base_bytes(int na) { return (sizeof(double2) + sizeof(float2)) * static_cast<size_t>(na); }
+inline size_t order_bytes(int na) { return sizeof(int) * kBpGroups + sizeof(uint16_t) * static_cast<size_t>(na); }
+inline size_t trig_bytes(int na) { return trig_base_bytes(na) + order_bytes(na); }
+// View of a table whose order sits elsewhere (null: behind the base arrays).
+inline Trig trig_view(void* table, int na, void* order = nullptr) {
+    Trig t;
+    t.cs = static_cast<const double2*>(table);
+    t.csf = reinterpret_cast<const float2*>(t.cs + na);
+    t.end = order ? static_cast<const int*>(order) : reinterpret_cast<const int*>(t.csf + na);
+    t.order = reinterpret_cast<const uint16_t*>(t.end + kBpGroups);
+    return t;
+}
 
 // Kernel launchers (implemented in the .cu files). Each returns the CUDA error
 // of the launch.
-cudaError_t launch_trig(const float* d_angles_deg, int na, double2* d_cs, cudaStream_t st);
+// Fills the cs, end and order arrays of an angle table from device degrees (the
+// order may overwrite the degrees).
+cudaError_t launch_trig(const float* d_angles_deg, int na, const Trig& t, cudaStream_t st);
 cudaError_t launch_slice_stats(const float* d_vol, long long npx, int nz, float4* d_stats,
                                cudaStream_t st, int4* d_box = nullptr, int2* d_band = nullptr,
                                int nband = 0);
@@ -194,7 +221,7 @@ cudaError_t launch_filter_gemm(const float* d_sino, int nz, int na, const PadGeo
 // result does not depend on what else shares the batch.
 constexpr int kMaxJobs = 64;
 
-// Backprojection job: items are (slice group, tile) pairs, slice-group major.
+// Backprojection job: items are (slice groups, tile) pairs, slice-group major.
 struct BpJob {
     const float4* filt;   // [nzg][na][pitch] float4
     float* out;           // [nz][n][n]
@@ -205,6 +232,7 @@ struct BpJob {
     int nz, na, sq, guard, pitch, n, denorm;
     int edge_rule;        // 1: SerialBackend's tap rule (both taps in range); 0: per-tap bounds
     int tiles_x, tiles;   // tiles per row / per slice group
+    int zgs;              // slice groups per item (1 or 2)
     long long first;      // index of the job's first item in the batch
 };
 struct BpBatch {
@@ -239,6 +267,9 @@ BpJob make_bp_job(const float4* d_filt, int nz, int na, const FiltLayout& fl, in
 FiltJob make_filt_job(const float* d_sino, int nz, int na, const PadGeom& g, const FiltLayout& fl,
                       const float2* d_Hc, const float4* d_stats, int denorm, float scale,
                       float4* d_filt);
+// Decide the slice groups per item of a batch (all of one tile shape) and number
+// its items: sets every job's zgs and first, and the total.
+void bp_number_items(BpBatch& b, int variant, int sms);
 // Backprojection of a batch (below 2^31 items, one tile shape): one CTA per
 // item, or with `persistent` a grid of resident CTAs drawing items from
 // d_counter (zeroed here on the stream). Filtering takes one CTA per item.

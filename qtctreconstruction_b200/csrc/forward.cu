@@ -21,6 +21,64 @@ __global__ void k_trig(const float* __restrict__ deg, int na, double2* __restric
     cs[a] = make_double2(c, s);
 }
 
+// The backprojector's angle order (Trig::order, Trig::end) by one block: a stable
+// counting sort of the angles by group. Each pass over blockDim angles counts or
+// places them by warp ballots, one lane per group.
+__global__ void __launch_bounds__(1024) k_bp_order(const double2* __restrict__ cs, int na, uint16_t* __restrict__ order,
+                                                   int* __restrict__ end) {
+    __shared__ int cnt[32][kBpGroups];  // per warp and group, then the warps' first positions
+    __shared__ int base[kBpGroups];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x < kBpGroups) base[threadIdx.x] = 0;
+    for (int place = 0; place < 2; ++place) {
+        for (int a0 = 0; a0 < na; a0 += 1024) {
+            const int a = a0 + threadIdx.x;
+            int key = -1;
+            if (a < na) {
+                const double2 t = cs[a];
+                const bool along_x = fabs(t.y) > fabs(t.x);
+                const double slow = along_x ? t.x : -t.y;  // u per voxel along the columns
+                const double m = fabs(slow);
+                key = (along_x ? 0 : 8) + (slow < 0.0 ? 4 : 0) +
+                      (m < 1.0 / 3.0 ? 0 : m < 0.5 ? 1 : m < 2.0 / 3.0 ? 2 : 3);
+            }
+            unsigned own = 0;
+#pragma unroll
+            for (int g = 0; g < kBpGroups; ++g) {
+                const unsigned m = __ballot_sync(0xffffffffu, key == g);
+                if (key == g) own = m;
+                if (lane == g) cnt[warp][g] = __popc(m);
+            }
+            __syncthreads();
+            if (threadIdx.x < kBpGroups) {
+                int run = base[threadIdx.x];
+                for (int w = 0; w < 32; ++w) {
+                    const int c = cnt[w][threadIdx.x];
+                    cnt[w][threadIdx.x] = run;
+                    run += c;
+                }
+                base[threadIdx.x] = run;
+            }
+            __syncthreads();
+            if (place && key >= 0)
+                order[cnt[warp][key] + __popc(own & ((1u << lane) - 1u))] = static_cast<uint16_t>(a);
+            __syncthreads();
+        }
+        if (!place) {  // group sizes to first positions
+            if (threadIdx.x == 0) {
+                int run = 0;
+                for (int g = 0; g < kBpGroups; ++g) {
+                    const int c = base[g];
+                    base[g] = run;
+                    run += c;
+                    end[g] = run;
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
 // ------------------------------------------------------------ slice stats
 // stats[z] = {min, max, span_fwd, span_denorm} (SerialBackend.cpp:70-80, 298-300).
 // With box set, also empties the non-zero bounding box of each 4-slice group
@@ -310,8 +368,9 @@ cudaError_t launch_raymarch(const float4* d_img, int w, int h, int nz, int na, i
     return cudaGetLastError();
 }
 
-cudaError_t launch_trig(const float* d_angles_deg, int na, double2* d_cs, cudaStream_t st) {
-    k_trig<<<(na + 127) / 128, 128, 0, st>>>(d_angles_deg, na, d_cs);
+cudaError_t launch_trig(const float* d_angles_deg, int na, const Trig& t, cudaStream_t st) {
+    k_trig<<<(na + 127) / 128, 128, 0, st>>>(d_angles_deg, na, const_cast<double2*>(t.cs));
+    k_bp_order<<<1, 1024, 0, st>>>(t.cs, na, const_cast<uint16_t*>(t.order), const_cast<int*>(t.end));
     return cudaGetLastError();
 }
 

@@ -124,14 +124,15 @@ extern "C" ctb_status ctb_fbp_noalloc(const float* d_sino, int depth, int num_an
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_csf, csf.data(), sizeof(float2) * num_angles, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_Hc, Hc.data(), sizeof(float2) * Hc.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = launch_trig(d_deg, num_angles, d_cs, st);
+    // once the degrees are read, their region takes the backprojector's angle order
+    static_assert(sizeof(int) * kBpGroups + sizeof(uint16_t) * kMaxAngles <= sizeof(float) * kMaxAngles,
+                  "the order fits the region of the degrees");
+    const Trig trig = trig_view(d_cs, num_angles, d_deg);
+    if (e == cudaSuccess) e = launch_trig(d_deg, num_angles, trig, st);
     const float scale = 3.14159265358979323846f / (2.0f * static_cast<float>(num_angles));
     if (e == cudaSuccess)
         e = launch_filter(d_sino, depth, num_angles, g, fl, d_Hc, d_tw, nullptr, CTB_DENORM_NONE, scale,
                           d_filt, st);
-    Trig trig;
-    trig.cs = d_cs;
-    trig.csf = d_csf;
     if (e == cudaSuccess)
         e = launch_backproject(d_filt, depth, num_angles, fl, output_size, trig, nullptr,
                                CTB_DENORM_NONE, d_out, d_err, st);

@@ -117,6 +117,7 @@ struct SReq {
     uint64_t seq = 0;
     ctb_request r{};
     std::vector<float> angles;
+    DevBuf order;            // the backprojector's angle order, a buffer of the server's pool
     State state = kPending;
     ctb_status status = CTB_ERR_BUSY;
     bool cancel = false;
@@ -179,6 +180,7 @@ struct ctb_server {
     std::mutex tables_mu;  // guards filters / twiddles (never held with mu)
     std::map<std::pair<int, int>, DevBuf> filters;
     std::map<int, DevBuf> twiddles;
+    std::vector<DevBuf> free_orders;  // angle-order buffers no request holds (guarded by mu)
     bool kick = false;     // something changed that may let a queued request in
     int inflight = 0;
     uint64_t batch_seq = 0;
@@ -205,7 +207,7 @@ void plan_request(SReq* q) {
     q->fl = filt_layout(q->g.sq, r.output_size);
     size_t off = 0;
     q->trig_off = off;
-    off += round_unit((sizeof(double2) + sizeof(float2)) * static_cast<size_t>(r.num_angles));
+    off += round_unit(trig_base_bytes(r.num_angles));
     q->filt_off = off;
     off += round_unit(sizeof(float4) * static_cast<size_t>((r.depth + 3) / 4) * r.num_angles * q->fl.pitch);
     q->sino_bytes = sizeof(float) * static_cast<size_t>(r.depth) * r.num_angles * r.bins;
@@ -227,6 +229,8 @@ void finalize(ctb_server* s, SReq* q, ctb_status st) {
         arena_free(&s->arena, q->off);
         q->has_block = false;
     }
+    if (q->order.ptr) s->free_orders.push_back(q->order);
+    q->order = DevBuf();
     q->state = kFinal;
     q->status = st;
     q->t_done = Clock::now();
@@ -279,6 +283,34 @@ ctb_status request_tables(ctb_server* s, SReq* q) {
     }
     q->Hc = static_cast<const float2*>(it->second.ptr);
     q->tw = static_cast<const float2*>(jt->second.ptr);
+    return CTB_OK;
+}
+
+// A device buffer for a request's angle order: one of the pool that is large
+// enough, else a new one (like the spectra, outside the memory budget; the pool
+// holds at most as many as requests were alive at once, and is freed with the
+// server). Called at submission, mu not held.
+ctb_status request_order(ctb_server* s, SReq* q) {
+    const size_t need = order_bytes(q->r.num_angles);
+    {
+        std::lock_guard<std::mutex> lk(s->mu);
+        for (DevBuf& b : s->free_orders)
+            if (b.bytes >= need) {
+                q->order = b;
+                b = s->free_orders.back();
+                s->free_orders.pop_back();
+                return CTB_OK;
+            }
+    }
+    size_t bytes = 8192;
+    while (bytes < need) bytes *= 2;
+    DevBuf b;
+    if (cudaMalloc(&b.ptr, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return CTB_ERR_OOM;
+    }
+    b.bytes = bytes;
+    q->order = b;
     return CTB_OK;
 }
 
@@ -357,16 +389,12 @@ ctb_status launch_batch(ctb_server* s, const std::vector<SReq*>& reqs, int slot)
         const int v = var[order[k]];
         while (k < n && bp.njobs < kMaxJobs && var[order[k]] == v) {
             const SReq* q = reqs[order[k]];
-            Trig trig;
-            trig.cs = static_cast<const double2*>(q->d_trig);
-            trig.csf = reinterpret_cast<const float2*>(static_cast<const double2*>(q->d_trig) + q->r.num_angles);
-            BpJob J = make_bp_job(q->d_filt, q->r.depth, q->r.num_angles, q->fl, q->r.output_size, trig, nullptr,
-                                  CTB_DENORM_NONE, q->d_out, v);
-            J.first = bp.total;
-            bp.total += static_cast<long long>(J.tiles) * ((J.nz + 3) / 4);
-            bp.job[bp.njobs++] = J;
+            const Trig trig = trig_view(q->d_trig, q->r.num_angles, q->order.ptr);
+            bp.job[bp.njobs++] = make_bp_job(q->d_filt, q->r.depth, q->r.num_angles, q->fl, q->r.output_size, trig, nullptr,
+                                             CTB_DENORM_NONE, q->d_out, v);
             ++k;
         }
+        bp_number_items(bp, v, s->sms);
         if (launch_backproject_batch(bp, v, s->d_err + 1, s->d_err, s->compute) != cudaSuccess) return CTB_ERR_CUDA;
     }
     if (cudaMemcpyAsync(s->h_err + slot, s->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, s->compute) !=
@@ -451,8 +479,9 @@ void CUDART_CB batch_done(void* p) {
     delete rec;
 }
 
-// Angle table: double2 cs via the device sincospi kernel from degrees staged in
-// the (not yet used) filtered-row region, then the reference's float cos/sin.
+// Angle table: double2 cs and the order via the device kernels from degrees
+// staged in the (not yet used) filtered-row region, and the reference's float
+// cos/sin.
 bool upload_trig(SReq* q, Stager& st) {
     const int na = q->r.num_angles;
     std::vector<float2> csf(na);
@@ -466,7 +495,7 @@ bool upload_trig(SReq* q, Stager& st) {
                cudaSuccess &&
            cudaMemcpyAsync(cs + na, csf.data(), sizeof(float2) * na, cudaMemcpyHostToDevice, st.stream) ==
                cudaSuccess &&
-           launch_trig(d_deg, na, cs, st.stream) == cudaSuccess &&
+           launch_trig(d_deg, na, trig_view(cs, na, q->order.ptr), st.stream) == cudaSuccess &&
            cudaStreamSynchronize(st.stream) == cudaSuccess;
 }
 
@@ -618,6 +647,7 @@ void free_server(ctb_server* s) {
     for (auto& st : s->down_st) free_stager(st);
     for (auto& kv : s->filters) cudaFree(kv.second.ptr);
     for (auto& kv : s->twiddles) cudaFree(kv.second.ptr);
+    for (auto& b : s->free_orders) cudaFree(b.ptr);
     if (s->d_base) cudaFree(s->d_base);
     if (s->d_err) cudaFree(s->d_err);
     if (s->h_err) cudaFreeHost(s->h_err);
@@ -743,12 +773,19 @@ ctb_status ctb_server_submit(ctb_server* s, const ctb_request* req, uint64_t* id
     q->r.angles_deg = nullptr;
     plan_request(q.get());
     if (q->bytes <= s->arena.capacity) {  // capacity is fixed at creation
-        std::lock_guard<std::mutex> tl(s->tables_mu);
-        const ctb_status st = request_tables(s, q.get());
+        {
+            std::lock_guard<std::mutex> tl(s->tables_mu);
+            const ctb_status st = request_tables(s, q.get());
+            if (st != CTB_OK) return st;
+        }
+        const ctb_status st = request_order(s, q.get());
         if (st != CTB_OK) return st;
     }
     std::lock_guard<std::mutex> lk(s->mu);
-    if (s->stop) return CTB_ERR_CANCELLED;
+    if (s->stop) {
+        if (q->order.ptr) s->free_orders.push_back(q->order);
+        return CTB_ERR_CANCELLED;
+    }
     if (q->bytes > s->arena.capacity) {
         ++s->rejected;
         return CTB_ERR_OOM;
