@@ -125,13 +125,13 @@ cudaError_t launch_raymarch(const float4* d_img, int w, int h, int nz, int na, i
 // same image rows at the same time. groups: {first index into order, count,
 // axis (0 rows, 1 columns), K}, K the output bins per strip of the group
 // (fwd_strip_bins of its smallest |kq|); max_strips = ceil(nd / smallest K).
-constexpr int kFwdRows = 16;   // walked rows per chunk (crossing in double once per chunk)
+constexpr int kFwdRows = 16;   // zero rows after the last image row
 constexpr int kFwdGroup = 4;   // angles per CTA
 constexpr int kFwdPlanes = 2;  // float4 image planes (4 slices each) per thread
 // Zero border of the normalised image planes: kFwdGuard pixels on both sides
 // of every row (the projector's windows reach at most 50 columns outside the
-// image) and kFwdRows rows after the last, so that every chunk the projector
-// walks reads inside the plane.
+// image) and kFwdRows rows after the last, so that every group of rows the
+// projector walks reads inside the plane.
 constexpr int kFwdGuard = 64;
 inline size_t fwd_plane_elems(int np, int nq) {
     return static_cast<size_t>(np + kFwdRows) * static_cast<size_t>(nq + 2 * kFwdGuard);

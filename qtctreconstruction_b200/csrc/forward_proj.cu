@@ -14,7 +14,7 @@
 // (rows when |cos| >= |sin|, else columns of the transposed copy). At walked
 // row p the strip's pixels are the 32 consecutive columns from the crossing
 // q*(p) of its lower bin edge: lane l owns column rint(q*) + S l (S the sign
-// of ds/dq), whose offset from the crossing is u = (l - phi) |kq| in bins,
+// of ds/dq), whose offset from the crossing is u = (l + phi) |kq| in bins,
 // phi = S (rint(q*) - q*) in [-1/2, 1/2]. So every row is one coalesced load
 // of 32 neighbouring pixels (each the 8 slices of a plane pair, 32 bytes, one
 // 256-bit load per lane), and lane l's pixel
@@ -26,14 +26,31 @@
 // angle group so that K + 1 <= 31.5 |kq|: the lanes' pixels cover the
 // strip's bins and the bin on either side.
 //
-// The crossing is evaluated in double once per chunk of PCH = 16 rows (an
-// integer column plus a float offset) and stepped in float within the chunk;
-// each 8-row half of a chunk is walked only where its lanes' columns meet the
-// non-zero pixels of that 8-row band. The warps of a CTA are the up to GMAX =
-// 4 angles of a group that share the walked axis, on the same strip index;
-// after one barrier that ends the set-up (per-angle constants from the plan's
-// FwdAngleRec table) they walk the same rows at nearly the same columns and
-// share the L1 lines, and never wait on one another again.
+// What a row needs beside the pixels is the same for all lanes: its column and
+// phi. So the warp prepares 32 rows at a time, lane r evaluating row r's crossing
+// in double and testing its 32 columns against the non-zero pixels of the row's
+// 8-row band; the walk then reads each row's two values from shared memory (one
+// broadcast) where every lane computing them for itself took 12 more
+// instructions per row. 8-row groups without a needed row are skipped. Reading
+// rows within one row of the range where the strip's columns, at most 31.5 wide,
+// come within kReach = 2 columns of the non-zero box (or of the image without
+// bounds), or at most 7 rows beyond it, with |dq*/dp| <= 1, the 32-column window
+// stays within 50 columns of the image on either side: inside the kFwdGuard = 64
+// border, which reads as zeros.
+//
+// Bound by the L1 data path (about 9 wavefronts per row of 1 KB, 74 % busy at 512^2
+// x 32 x 720 without zeros) and issue (28 instructions per row, 12 of them packed
+// FP32x2 of two issue cycles): 5.56 -> 4.51 ms at 512^3 x 720 of the benchmark
+// phantom, 3.00 -> 2.53 ms at 512^2 x 64 x 720 without zeros, against each lane
+// preparing its rows. Measured there and not kept: 16 slices per lane (3.53 ms), 8
+// angles per CTA (2.92), 6 or 8 CTAs per SM (2.77, 3.37), four rows' loads ahead
+// (2.55), prefetching the next rows into L1 (2.61), saturating weights (2.54).
+//
+// The warps of a CTA are the up to GMAX = 4 angles of a group that share the
+// walked axis, on the same strip index; after one barrier that ends the set-up
+// (per-angle constants from the plan's FwdAngleRec table) they walk the same rows
+// at nearly the same columns and share the L1 lines, and never wait on one
+// another again.
 // Bins 0 and nd-1 are recomputed by the warp whose strip holds them, with one
 // lane per row deciding on the reference's own float s for the few pixels
 // around those bins.
@@ -46,21 +63,18 @@ namespace ctb {
 namespace {
 
 constexpr int LANES = 32;
-constexpr int PCH = kFwdRows;
+constexpr int PCH = kFwdRows;  // zero rows below the image
 constexpr int GMAX = kFwdGroup;
 constexpr int THREADS = LANES * GMAX;
 constexpr int NP = kFwdPlanes;          // float4 planes (4 slices each) per thread
-constexpr float kRound = 12582912.0f;   // 1.5 * 2^23: x + kRound rounds x to an integer
-constexpr int kRoundBits = 0x4B400000;  // bit pattern of kRound
-static_assert(kFwdGuard >= 50, "the walked windows reach 50 columns outside the image (see strip_rows)");
-static_assert(PCH == 16, "a chunk is two 8-row bands of the non-zero bounds");
+static_assert(kFwdGuard >= 50, "the walked windows reach 50 columns outside the image");
+static_assert(PCH >= 8, "an 8-row group may start at the image's last row");
 static_assert(NP == 2, "a pixel holds the 8 slices of a plane pair: two float4, one 32-byte load");
 
 struct FAngle {
     double q0;   // crossing of the strip's lower edge (bin b_lo = k K - 1) at p = 0
     double inv;  // dq*/db = 1 / kq
     double dq;   // dq*/dp = -kp / kq
-    float dqf;
     float akq;     // |kq|: bins per pixel step along the walked row
     float cf, sf;  // the reference's float cos/sin
     int a;
@@ -85,37 +99,24 @@ __device__ __forceinline__ int lane_bin(int l, float akq) {
     return static_cast<int>(floorf((static_cast<float>(l) - 0.5f) * akq));
 }
 
-// One chunk of the walk. Row pp crosses the strip's lower edge at column
-// base + A, A = fa + pp dq (float); the lanes read columns cb + S l, cb =
-// base + rint(A). With phi = S (rint(A) - A), lane l's pixel lies u = (l -
-// phi) |kq| bins above the edge, and y = u - m_l - 1 = cl1 - phi |kq| (cl1 =
-// l |kq| - m_l - 1) in [-1, 1] gives its hat weights for bins m_l, m_l + 1,
-// m_l + 2: max(-y, 0), 1 - |y|, max(y, 0).
-// Reads stay inside the zero border: a walked row lies within one row of the
-// range where the strip's columns, at most 31.5 wide, come within kReach = 2
-// columns of the non-zero box (or of the image without bounds), or at most 15
-// rows beyond it (chunks start on multiples of 16), and |dq| <= 1. So the
-// window start is at least 2 + 1 + 31.5 + 0.5 + 15 = 50 columns left of the
-// box's first column and at most 2 + 1 + 0.5 + 15 = 18.5 right of its last
-// (mirrored for S < 0), and the 32-column window stays within 50 columns of
-// the image on either side: inside the kFwdGuard = 64 border, which reads as
-// zeros.
-// Rows P0 .. P0 + NR - 1 of the chunk.
-template <int S, int P0, int NR>
-__device__ __forceinline__ void strip_rows(const float4* __restrict__ rowp, int pitch, int base, float fa,
-                                           float dqf, float akq, float cl1, int lane, float2 (&acc)[3][2 * NP]) {
+// One walked row of the strip, as one lane prepares it for the warp.
+struct RowRec {
+    float dy;      // S (rint(q*) - q*) |kq|: the pixels' offset from their nominal place, in bins
+    unsigned col;  // pixel index of column rint(q*) from the block's first row, left border included
+};
+
+// Eight rows of a block. Lane l's pixel of a row lies y = cl1 + dy bins from bin
+// m_l + 1 (cl1 = l |kq| - m_l - 1), y in [-1, 1], which gives its hat weights
+// for bins m_l, m_l + 1, m_l + 2: max(-y, 0), 1 - |y|, max(y, 0).
+__device__ __forceinline__ void walk_rows(const float4* __restrict__ lane_base, const RowRec* __restrict__ rr,
+                                          float cl1, float2 (&acc)[3][2 * NP]) {
 #pragma unroll
-    for (int pp = P0; pp < P0 + NR; ++pp) {
-        const float A = fmaf(static_cast<float>(pp), dqf, fa);
-        const float tr = A + kRound;
-        const float rr = tr - kRound;
-        const int cb = base + (__float_as_int(tr) - kRoundBits);
-        const float y = fmaf(S > 0 ? rr - A : A - rr, akq, cl1);
+    for (int i = 0; i < 8; ++i) {
+        const float y = cl1 + rr[i].dy;
         const float w0 = fmaxf(-y, 0.0f), w2 = fmaxf(y, 0.0f), w1 = 1.0f - fabsf(y);
         const float2 W0 = make_float2(w0, w0), W1 = make_float2(w1, w1), W2 = make_float2(w2, w2);
-        const float4* px = rowp + 2 * (static_cast<long long>(pp) * pitch + cb + S * lane);
         float4 v[NP];
-        ld_pixel(px, v);
+        ld_pixel(lane_base + 2ull * rr[i].col, v);
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
             acc[0][2 * k] = __ffma2_rn(W0, lo2(v[k]), acc[0][2 * k]);
@@ -188,6 +189,7 @@ __global__ void __launch_bounds__(THREADS, 7) k_forward(const float4* __restrict
                                                         float* __restrict__ sino) {
     __shared__ FAngle fa[GMAX];
     __shared__ int erow[GMAX][4];                      // edge-pass rows: bin 0 [lo, hi], bin nd-1 [lo, hi]
+    __shared__ __align__(16) RowRec rows_sm[GMAX][LANES];  // the block of rows each warp walks
 
     const int4 grp = groups[blockIdx.y];
     const int cnt = grp.y;
@@ -248,7 +250,6 @@ __global__ void __launch_bounds__(THREADS, 7) k_forward(const float4* __restrict
         f.inv = R.inv;
         f.dq = -kp * f.inv;
         f.q0 = cq + (static_cast<double>(b_lo) - dcf + cp * kp) * f.inv;
-        f.dqf = static_cast<float>(f.dq);
         f.akq = static_cast<float>(fabs(kq));
         f.neg = kq < 0.0 ? 1 : 0;
         f.cf = R.cf;
@@ -332,48 +333,44 @@ __global__ void __launch_bounds__(THREADS, 7) k_forward(const float4* __restrict
         const float akq = f.akq;
         const int ml = lane_bin(lane, akq);
         const float cl1 = fmaf(static_cast<float>(lane), akq, -static_cast<float>(ml + 1));
-        // chunks start on multiples of PCH, so that warps whose row ranges
-        // overlap walk the same rows at about the same time; each half of a
-        // chunk is then exactly one 8-row band
-        for (int p0 = f.p_lo & ~(PCH - 1); p0 <= f.p_hi; p0 += PCH) {
-            const double qs = fma(static_cast<double>(p0), f.dq, f.q0);
-            const double qfl = floor(qs);
-            const int base = static_cast<int>(qfl);
-            const float fq = static_cast<float>(qs - qfl);
-            // Each half walks only when the columns its lanes read, base +
-            // rint(fq + pp dqf) + S l with fq in [0, 1), meet its non-zero
-            // columns: the range of its band over the CTA's slice groups
-            // (none for rows past the image), or the box without bands. A
-            // skipped half adds only zeros.
-            bool walk[2];
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                int cl = f.c_lo, ch = f.c_hi;
-                if (band) {
-                    cl = INT_MAX;
-                    ch = -1;
-                    const int bi = (p0 >> 3) + hh;
-                    for (int k = 0; k < NP && bi < nb_p; ++k) {
-                        if (g0 + k >= ng4) break;
-                        const int2 r = __ldg(band + static_cast<long long>(g0 + k) * nb_all + nb_off + bi);
-                        cl = min(cl, r.x);
-                        ch = max(ch, r.y);
-                    }
+        RowRec* rr = rows_sm[ja];
+        // blocks start on multiples of 32 rows, so that warps whose row ranges
+        // overlap walk the same rows at about the same time
+        for (int p0 = f.p_lo & ~(LANES - 1); p0 <= f.p_hi; p0 += LANES) {
+            // lane r prepares row p0 + r: its crossing in double, and whether
+            // the 32 columns from there meet the row's non-zero columns (the
+            // range of its 8-row band over the CTA's slice groups, none past the
+            // image; or the box without bands)
+            const int p = p0 + lane;
+            const double q = fma(static_cast<double>(p), f.dq, f.q0);
+            const double qr = rint(q);
+            const int col = static_cast<int>(qr);
+            const float d = static_cast<float>(qr - q);
+            int cl = f.c_lo, ch = f.c_hi;
+            if (band) {
+                cl = INT_MAX;
+                ch = -1;
+                const int bi = p >> 3;
+                for (int k = 0; k < NP && bi < nb_p; ++k) {
+                    if (g0 + k >= ng4) break;
+                    const int2 r = __ldg(band + static_cast<long long>(g0 + k) * nb_all + nb_off + bi);
+                    cl = min(cl, r.x);
+                    ch = max(ch, r.y);
                 }
-                const float e0 = static_cast<float>(8 * hh) * f.dqf, e1 = static_cast<float>(8 * hh + 7) * f.dqf;
-                const int lo = base + static_cast<int>(floorf(fminf(e0, e1))) - 1 - (f.neg ? LANES - 1 : 0);
-                const int hi = base + static_cast<int>(ceilf(fmaxf(e0, e1))) + 2 + (f.neg ? 0 : LANES - 1);
-                walk[hh] = ch >= cl && hi >= cl && lo <= ch;
             }
-            const bool w0 = walk[0], w1 = walk[1];
-            const float4* rowp = plane + 2LL * p0 * pitch;
-            if (f.neg) {
-                if (w0) strip_rows<-1, 0, 8>(rowp, pitch, base, fq, f.dqf, akq, cl1, lane, acc);
-                if (w1) strip_rows<-1, 8, 8>(rowp, pitch, base, fq, f.dqf, akq, cl1, lane, acc);
-            } else {
-                if (w0) strip_rows<1, 0, 8>(rowp, pitch, base, fq, f.dqf, akq, cl1, lane, acc);
-                if (w1) strip_rows<1, 8, 8>(rowp, pitch, base, fq, f.dqf, akq, cl1, lane, acc);
-            }
+            const int first = f.neg ? col - (LANES - 1) : col;
+            const unsigned need = __ballot_sync(
+                0xffffffffu, p >= f.p_lo && p <= f.p_hi && ch >= cl && first + LANES - 1 >= cl && first <= ch);
+            if (!need) continue;
+            __syncwarp();  // the last block's rows are read
+            rr[lane] = RowRec{(f.neg ? -d : d) * akq, static_cast<unsigned>(lane * pitch + col + kFwdGuard)};
+            __syncwarp();
+            const float4* lane_base =
+                plane + 2 * (static_cast<long long>(p0) * pitch - kFwdGuard + (f.neg ? -lane : lane));
+            // groups of 8 rows without a needed one add only zeros
+#pragma unroll 1
+            for (int g = 0; g < LANES; g += 8)
+                if ((need >> g) & 0xffu) walk_rows(lane_base, rr + g, cl1, acc);
         }
     }
     if (!has_a) return;

@@ -1,0 +1,48 @@
+"""The forward projector's blocks of 32 prepared rows on the GPU.
+
+Image heights around the blocks' and the 8-row groups' ends, non-zero regions
+that leave rows, groups and whole blocks out, and slice counts around the 8
+slices a warp holds, with the non-zero bounds on and off, against the FP64
+oracle at the projector's parity bar.
+"""
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bounds", [True, False])
+@pytest.mark.parametrize("n,depth", [(7, 1), (31, 9), (33, 2), (64, 8), (71, 17)])
+@pytest.mark.parametrize("region", ["full", "one_pixel", "corner", "two_bands"])
+def test_rows_meet_parity(backend, region, n, depth, bounds):
+    import torch
+    rng = np.random.default_rng(n + depth)
+    vol = rng.uniform(0.5, 1.5, (depth, n, n)).astype(np.float32)
+    keep = np.zeros((n, n), bool)
+    if region == "full":
+        keep[:] = True
+    elif region == "one_pixel":
+        keep[n // 2, n // 3] = True
+    elif region == "corner":
+        keep[: max(1, n // 8), n - max(1, n // 8):] = True
+    else:
+        keep[n // 9, :] = keep[n - 1 - n // 7, n // 2:] = True
+    vol[:, ~keep] = 0.0
+    na, nd = 23, (3 * n) // 2 + 1
+    ang = (np.arange(na) * 111.246117975 % 180.0).astype(np.float32)
+    d_v = torch.from_numpy(vol).cuda()
+    d_s = torch.full((depth, na, nd), float("nan"), device="cuda")
+    d_st = torch.empty(depth, 4, device="cuda")
+    backend.set_forward_bounds(bounds)
+    try:
+        backend.forward_d(d_v.data_ptr(), n, depth, na, nd, d_s.data_ptr(), d_st.data_ptr(), ang)
+        backend.synchronize()
+    finally:
+        backend.set_forward_bounds(True)
+    got = d_s.cpu().numpy()
+    for z in range(depth):
+        ref = O.sinogram_f64(vol[z], na, nd, ang)[0]
+        assert np.all(np.isfinite(got[z]))
+        assert np.linalg.norm(got[z] - ref) <= 1e-5 * max(np.linalg.norm(ref), 1e-30) + 1e-12
