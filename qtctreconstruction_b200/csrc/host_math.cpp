@@ -230,26 +230,32 @@ void generator3d_boxes(const float* ell, int count, int nx, int ny, int nz, floa
 namespace ctb {
 
 // Group the projection angles for the forward projector: angles are split by
-// walked axis (|cos| >= |sin| walks rows, else columns), kept in their given
-// order within each axis, and cut into groups of kFwdGroup consecutive
-// angles, which walk nearly the same rows and columns and so share L1 lines.
+// walked axis (|cos| >= |sin| walks rows, else columns), sorted by direction
+// within each axis, and cut into groups of kFwdGroup neighbours, which walk
+// nearly the same rows and columns and so share L1 lines whatever the order of
+// the list (450 angles in golden-angle order at 300^2 x 37: 497 -> 415 us).
 FwdPlan forward_plan(const float* angles_deg, int na, int w, int h, int nd) {
     (void)w;
     (void)h;
     std::vector<int> lists[2];
-    std::vector<double> akq(na);
+    std::vector<double> akq(na), slope(na);
     for (int a = 0; a < na; ++a) {
         // the projector's own trig (k_trig): sincospi of deg / 180 in double
         const double t = static_cast<double>(angles_deg[a]) / 180.0;
-        const double c = std::fabs(std::cos(3.14159265358979323846 * t));
-        const double s = std::fabs(std::sin(3.14159265358979323846 * t));
+        const double cs = std::cos(3.14159265358979323846 * t), sn = std::sin(3.14159265358979323846 * t);
+        const double c = std::fabs(cs), s = std::fabs(sn);
         const int axis = c >= s ? 0 : 1;
         akq[a] = axis == 0 ? c : s;
+        // the walked direction's slope, in [-1, 1]: neighbours on either axis
+        // (an angle that is not finite has no direction: anywhere in the order)
+        slope[a] = axis == 0 ? sn / cs : cs / sn;
+        if (!std::isfinite(slope[a])) slope[a] = 0.0;
         lists[axis].push_back(a);
     }
     FwdPlan plan;
     for (int axis = 0; axis < 2; ++axis) {
-        const auto& L = lists[axis];
+        auto& L = lists[axis];
+        std::stable_sort(L.begin(), L.end(), [&](int x, int y) { return slope[x] < slope[y]; });
         for (size_t i = 0; i < L.size(); i += kFwdGroup) {
             const int first = static_cast<int>(plan.order.size());
             const int cnt = static_cast<int>(std::min<size_t>(kFwdGroup, L.size() - i));
