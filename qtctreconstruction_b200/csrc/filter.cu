@@ -688,21 +688,43 @@ __device__ __forceinline__ void passes16p(float4* buf, int j, const float4* __re
     }
 }
 
-// Lengths up to kPackedMaxL = 2048, registers held to 128 (four CTAs per SM
-// at 2048, no spills; a 96-register cap for a fifth CTA spills and measured
-// slower, 1.81 against 1.56 ms at 512^3 x 720). At 4096 the 16 pairs per
-// thread need more than 128 registers (one 256-thread CTA per SM) and the
-// kernel is slower than the scalar one (5.35 against 4.68 ms at 1024^2 x 256 x
-// 1440), which therefore keeps lengths 4096 and 8192.
+// Lengths up to kPackedMaxL = 2048, registers held to 128 from length 512 on (four
+// CTAs per SM at 2048, eight at 1024, sixteen at 512). Bounding every length to
+// four CTAs only let the compiler take 186 and 194 registers at 1024 and 512 and
+// left 10 warps per SM: 84.9 -> 70.4 us at 387^2 x 50 x 580, 56.8 -> 50.4 us at
+// 200^2 x 64 x 314 with the bound, and a 96-register cap is slower again (76.2 and
+// 54.6 us; at 2048 208 against 188 us). Below 512 several items share a warp (48^2 x
+// 200 x 80: FBP 47.1 -> 39.8 us). At 4096 the 16 pairs per thread need more than
+// 128 registers (one 256-thread CTA per SM) and the kernel is slower than the
+// scalar one (5.35 against 4.68 ms at 1024^2 x 256 x 1440), which therefore keeps
+// lengths 4096 and 8192.
+//
+// CTA of k_filter4: T = L/16 threads per item, at least one warp (several items
+// below length 512).
+constexpr int filter4_items(int logl) { return logl >= 9 ? 1 : 1 << (9 - logl); }
+constexpr int filter4_threads(int logl) { return logl >= 9 ? (1 << logl) / 16 : 32; }
+// float4 elements of an item in shared memory: at length 64 two items share an
+// 8-lane phase and sit half a bank row apart
+constexpr int filter4_stride(int logl) { return (1 << logl) + (logl == 6 ? 4 : 0); }
+// Threads per SM the registers are held to: 512 (128 registers) from length 512
+// on, 256 below, where the compiler's own allocation is short of spilling (at 512
+// threads 24.6 against 22.6 us for an FBP of 64^2 x 16 x 101).
+constexpr int filter4_resident(int logl) { return logl >= 9 ? 512 : 256; }
 template <int LOGL>
-__global__ void __launch_bounds__((1 << LOGL) / 16, 4) k_filter4(const __grid_constant__ FiltBatch batch) {
+__global__ void __launch_bounds__(filter4_threads(LOGL), filter4_resident(LOGL) / filter4_threads(LOGL))
+    k_filter4(const __grid_constant__ FiltBatch batch) {
     constexpr int L = 1 << LOGL, T = L / 16, REM = LOGL & 3, Q = LOGL >> 2;
+    constexpr int ITEMS = filter4_items(LOGL);
     constexpr int R0 = REM ? (1 << REM) : 16;  // radix of the first and the last pass
     constexpr int NB0 = 16 / R0;               // their butterflies per thread
     constexpr int FWD16 = Q - 1 - (REM == 0 ? 1 : 0);
-    extern __shared__ float4 smem4[];
-    const long long item = blockIdx.x + static_cast<long long>(blockIdx.y) * gridDim.x;
-    if (item >= batch.total) return;
+    extern __shared__ float4 smem_all[];
+    const long long first = (blockIdx.x + static_cast<long long>(blockIdx.y) * gridDim.x) * ITEMS;
+    if (first >= batch.total) return;
+    // places past the last item repeat it (the same values to the same bins)
+    const int place = ITEMS > 1 ? threadIdx.x / T : 0;
+    const long long item = ITEMS > 1 ? min(first + place, batch.total - 1) : first;
+    float4* smem4 = smem_all + place * filter4_stride(LOGL);
     int jb = 0;
     while (jb + 1 < batch.njobs && batch.job[jb + 1].first <= item) ++jb;
     const FiltJob& J = batch.job[jb];
@@ -711,7 +733,7 @@ __global__ void __launch_bounds__((1 << LOGL) / 16, 4) k_filter4(const __grid_co
     const int a = static_cast<int>(local % na);
     const int zg = static_cast<int>(local / na);
     const int z0 = 4 * zg;
-    const int tid = threadIdx.x;
+    const int tid = ITEMS > 1 ? threadIdx.x % T : threadIdx.x;
     const float* rows[4];
 #pragma unroll
     for (int s = 0; s < 4; ++s)
@@ -886,18 +908,19 @@ FiltJob make_filt_job(const float* d_sino, int nz, int na, const PadGeom& g, con
 
 template <int LOGL>
 cudaError_t launch_filter4(const FiltBatch& b, cudaStream_t st) {
-    constexpr int L = 1 << LOGL;
-    const size_t smem = sizeof(float4) * L;
+    constexpr int ITEMS = filter4_items(LOGL);
+    const size_t smem = sizeof(float4) * ITEMS * filter4_stride(LOGL);
     cudaError_t e = cudaFuncSetAttribute(k_filter4<LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem));
     // (no shared-memory carveout preference: the twiddle and spectrum tables
     // are read through L1, and a full carveout measured slower, 1.71 ms
     // against 1.56 ms at 512^3 x 720)
     if (e != cudaSuccess) return e;
-    const long long gx = b.total < 65535 ? b.total : 65535;
-    const long long gy = (b.total + gx - 1) / gx;
+    const long long ctas = (b.total + ITEMS - 1) / ITEMS;
+    const long long gx = ctas < 65535 ? ctas : 65535;
+    const long long gy = (ctas + gx - 1) / gx;
     if (gy > 65535) return cudaErrorInvalidValue;
-    k_filter4<LOGL><<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), L / 16, smem, st>>>(b);
+    k_filter4<LOGL><<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), filter4_threads(LOGL), smem, st>>>(b);
     return cudaGetLastError();
 }
 
