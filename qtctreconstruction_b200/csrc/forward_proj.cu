@@ -179,14 +179,18 @@ __device__ __noinline__ void edge_bin(const float4* __restrict__ plane, int pitc
         }
 }
 
-__global__ void __launch_bounds__(THREADS, 7) k_forward(const float4* __restrict__ img,
-                                                        const float4* __restrict__ imgT, int w,
-                                                        int h, int nz, int na, int nd,
-                                                        const int4* __restrict__ groups,
-                                                        const FwdAngleRec* __restrict__ arec,
-                                                        const int4* __restrict__ box,
-                                                        const int2* __restrict__ band,
-                                                        float* __restrict__ sino) {
+// PER_SM: the CTAs per SM the registers are held to. Seven (72 registers) for
+// launches that fill the SMs. A launch that does not is bound by the latency of its
+// loads: four per SM (127 registers) let a warp have all eight rows of a group on
+// their way (us of a whole call, seven against four: 45.1 and 33.4 at 160^2 x 1 x
+// 180, 39.0 and 29.8 at 128^2 x 8 x 180, 28.7 and 22.6 at 64^2 x 1 x 90; but 72.0
+// and 73.3 at 256^2 x 1 x 360 with 1620 CTAs, 2563 and 2714 at 512^2 x 64 x 720).
+constexpr int FULL = 7, SPARSE = 4;
+template <int PER_SM>
+__global__ void __launch_bounds__(THREADS, PER_SM)
+    k_forward(const float4* __restrict__ img, const float4* __restrict__ imgT, int w, int h, int nz, int na, int nd,
+              const int4* __restrict__ groups, const FwdAngleRec* __restrict__ arec, const int4* __restrict__ box,
+              const int2* __restrict__ band, float* __restrict__ sino) {
     __shared__ FAngle fa[GMAX];
     __shared__ int erow[GMAX][4];                      // edge-pass rows: bin 0 [lo, hi], bin nd-1 [lo, hi]
     __shared__ __align__(16) RowRec rows_sm[GMAX][LANES];  // the block of rows each warp walks
@@ -466,8 +470,13 @@ cudaError_t launch_forward(const float4* d_img, const float4* d_imgT, int w, int
                            const FwdAngleRec* d_rec, const int4* d_box, const int2* d_band, float* d_sino,
                            cudaStream_t st) {
     const dim3 grid(max_strips, ngroups, ((nz + 3) / 4 + NP - 1) / NP);
-    k_forward<<<grid, dim3(LANES, GMAX), 0, st>>>(d_img, d_imgT, w, h, nz, na, nd, d_groups, d_rec, d_box,
-                                                  d_band, d_sino);
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const bool sparse = static_cast<long long>(grid.x) * grid.y * grid.z <= static_cast<long long>(SPARSE) * sms;
+    auto kernel = sparse ? k_forward<SPARSE> : k_forward<FULL>;
+    kernel<<<grid, dim3(LANES, GMAX), 0, st>>>(d_img, d_imgT, w, h, nz, na, nd, d_groups, d_rec, d_box, d_band,
+                                               d_sino);
     return cudaGetLastError();
 }
 
