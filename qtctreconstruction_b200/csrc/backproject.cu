@@ -628,6 +628,7 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
         S.dead = 0;
         mbar_fence_init();
     }
+    chain_wait();  // lets the next call's first kernel start in this one's tail
     unsigned stages = 0;
     if constexpr (MODE == 0) {
         __syncthreads();
@@ -674,6 +675,11 @@ cudaError_t set_smem() {
     return e;
 }
 
+// These launches wait for the kernel before them to end (they are not chained):
+// blocks that start while the filter's last ones still hold their SMs pile up on
+// the SMs that are free first, and stay there for the whole angle loop (194
+// against 162 us for a volume of 128^3 x 180, 225 against 197 us for a slice of
+// 256^2 x 360).
 template <class C>
 cudaError_t launch_one(const BpBatch& b, unsigned* d_err, cudaStream_t st) {
     cudaError_t e = set_smem<C>();

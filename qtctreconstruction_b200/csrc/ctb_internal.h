@@ -105,6 +105,35 @@ inline Trig trig_view(void* table, int na, void* order = nullptr) {
     return t;
 }
 
+// Launch of a kernel that may start while the kernel before it in the stream
+// ends (programmatic dependent launch). Such a kernel calls chain_wait before it
+// reads or writes global memory: from there on every earlier kernel of the stream
+// is complete and its writes are visible. chain_wait then lets the next kernel's
+// blocks start, once all of this kernel's have. Measured, us per call: 23.6 -> 19.0
+// for an FBP of 64^2 x 16 x 101, 415 -> 404 for a forward projection of 300^2 x 37 x
+// 450, 32.8 -> 27.2 of 160^2 x 1 x 180.
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                  A&&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 // Kernel launchers (implemented in the .cu files). Each returns the CUDA error
 // of the launch.
 // Fills the cs, end and order arrays of an angle table from device degrees (the

@@ -449,6 +449,7 @@ __global__ void __launch_bounds__(256, (K == 1 ? 3 : 1)) k_filter(const __grid_c
     const int z0 = 2 * static_cast<int>(local / na), z1 = z0 + 1;
     const int T = blockDim.x;
     const int tid = threadIdx.x;
+    chain_wait();
     const float* r0 = J.sino + (static_cast<long long>(z0) * na + a) * nd;
     const float* r1 = z1 < nz ? J.sino + (static_cast<long long>(z1) * na + a) * nd : nullptr;
     // rows z0, z1 are lanes (z0 % 4, z0 % 4 + 1) of the float4 layout
@@ -734,6 +735,7 @@ __global__ void __launch_bounds__(filter4_threads(LOGL), filter4_resident(LOGL) 
     const int zg = static_cast<int>(local / na);
     const int z0 = 4 * zg;
     const int tid = ITEMS > 1 ? threadIdx.x % T : threadIdx.x;
+    chain_wait();
     const float* rows[4];
 #pragma unroll
     for (int s = 0; s < 4; ++s)
@@ -920,8 +922,8 @@ cudaError_t launch_filter4(const FiltBatch& b, cudaStream_t st) {
     const long long gx = ctas < 65535 ? ctas : 65535;
     const long long gy = (ctas + gx - 1) / gx;
     if (gy > 65535) return cudaErrorInvalidValue;
-    k_filter4<LOGL><<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), filter4_threads(LOGL), smem, st>>>(b);
-    return cudaGetLastError();
+    return launch_chained(k_filter4<LOGL>, dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)),
+                          filter4_threads(LOGL), smem, st, b);
 }
 
 cudaError_t launch_filter_batch(const FiltBatch& b, cudaStream_t st) {
@@ -959,8 +961,7 @@ cudaError_t launch_filter_batch(const FiltBatch& b, cudaStream_t st) {
     const long long gx = b.total < 65535 ? b.total : 65535;
     const long long gy = (b.total + gx - 1) / gx;
     if (gy > 65535) return cudaErrorInvalidValue;
-    kern<<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), threads, smem, st>>>(b, logL);
-    return cudaGetLastError();
+    return launch_chained(kern, dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), threads, smem, st, b, logL);
 }
 
 cudaError_t launch_filter(const float* d_sino, int nz, int na, const PadGeom& g,

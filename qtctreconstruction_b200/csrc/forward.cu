@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(1024) k_slice_stats(const float* __restrict__ 
                                                       float4* __restrict__ stats, int4* __restrict__ box,
                                                       int2* __restrict__ band, int nband) {
     const int z = blockIdx.x;
+    chain_wait();
     if (box && threadIdx.x == 0 && (z & 3) == 0) {
         box[2 * (z >> 2)] = make_int4(INT_MAX, -1, INT_MAX, -1);
         box[2 * (z >> 2) + 1] = make_int4(-1, 0, 0, 0);
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(256) k_normalize(const float* __restrict__ vol
     if (zg >= (nz + 3) / 4) return;  // a pair with one group (uniform per block)
     const int x0 = (blockIdx.x >> 1) * 32, y0 = blockIdx.y * 32;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+    chain_wait();
     float lo[4], inv[4];
     bool live[4];
 #pragma unroll
@@ -302,6 +304,7 @@ __global__ void __launch_bounds__(128) k_raymarch(const float4* __restrict__ img
     const int a = blockIdx.y;
     const int zg = blockIdx.z;
     if (b >= nd) return;
+    chain_wait();
     const long long pitch = w + 2 * kFwdGuard;
     // group zg is half zg % 2 of the pixels (two float4 each) of plane pair zg / 2
     const float4* plane = img + static_cast<long long>(zg / 2) * (h + kFwdRows) * pitch * 2 + 2 * kFwdGuard + (zg & 1);
@@ -364,8 +367,7 @@ __global__ void __launch_bounds__(128) k_raymarch(const float4* __restrict__ img
 cudaError_t launch_raymarch(const float4* d_img, int w, int h, int nz, int na, int nd, float det_center,
                             const double2* d_cs, float* d_sino, cudaStream_t st) {
     const dim3 grid((nd + 127) / 128, na, (nz + 3) / 4);
-    k_raymarch<<<grid, 128, 0, st>>>(d_img, w, h, nz, na, nd, det_center, d_cs, d_sino);
-    return cudaGetLastError();
+    return launch_chained(k_raymarch, grid, 128, 0, st, d_img, w, h, nz, na, nd, det_center, d_cs, d_sino);
 }
 
 cudaError_t launch_trig(const float* d_angles_deg, int na, const Trig& t, cudaStream_t st) {
@@ -376,16 +378,15 @@ cudaError_t launch_trig(const float* d_angles_deg, int na, const Trig& t, cudaSt
 
 cudaError_t launch_slice_stats(const float* d_vol, long long npx, int nz, float4* d_stats,
                                cudaStream_t st, int4* d_box, int2* d_band, int nband) {
-    k_slice_stats<<<nz, 1024, 0, st>>>(d_vol, npx, d_stats, d_box, d_band, nband);
-    return cudaGetLastError();
+    return launch_chained(k_slice_stats, nz, 1024, 0, st, d_vol, npx, d_stats, d_box, d_band, nband);
 }
 
 cudaError_t launch_normalize(const float* d_vol, int w, int h, int nz, const float4* d_stats,
                              float4* d_img, float4* d_imgT, cudaStream_t st, int skip_zero,
                              int4* d_box, int2* d_band) {
     const dim3 grid(2 * ((w + 31) / 32), (h + 31) / 32, (nz + 7) / 8);
-    k_normalize<<<grid, 256, 0, st>>>(d_vol, w, h, nz, d_stats, d_img, d_imgT, skip_zero, d_box, d_band);
-    return cudaGetLastError();
+    return launch_chained(k_normalize, grid, 256, 0, st, d_vol, w, h, nz, d_stats, d_img, d_imgT, skip_zero, d_box,
+                          d_band);
 }
 
 }  // namespace ctb

@@ -200,6 +200,7 @@ __global__ void __launch_bounds__(THREADS, PER_SM)
     const bool rows = grp.z == 0;
     const int K = grp.w;  // output bins per strip for this group
     if (blockIdx.x * K >= nd) return;  // the group has fewer strips than the grid (uniform per CTA)
+    chain_wait();
     const int b_lo = blockIdx.x * K - 1;       // the strip's lower edge bin
     const int nout = min(K, nd - 1 - b_lo);    // output bins b_lo + 1 .. b_lo + nout
     const bool has0 = b_lo < 0, has_last = b_lo + nout == nd - 1;
@@ -474,10 +475,8 @@ cudaError_t launch_forward(const float4* d_img, const float4* d_imgT, int w, int
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const bool sparse = static_cast<long long>(grid.x) * grid.y * grid.z <= static_cast<long long>(SPARSE) * sms;
-    auto kernel = sparse ? k_forward<SPARSE> : k_forward<FULL>;
-    kernel<<<grid, dim3(LANES, GMAX), 0, st>>>(d_img, d_imgT, w, h, nz, na, nd, d_groups, d_rec, d_box, d_band,
-                                               d_sino);
-    return cudaGetLastError();
+    return launch_chained(sparse ? k_forward<SPARSE> : k_forward<FULL>, grid, dim3(LANES, GMAX), 0, st, d_img, d_imgT, w,
+                          h, nz, na, nd, d_groups, d_rec, d_box, d_band, d_sino);
 }
 
 cudaError_t launch_fwd_angles(const int4* d_groups, int ngroups, const int* d_order, Trig trig,
