@@ -222,11 +222,17 @@ ctb_status forward_plan_dev(ctb_ctx* ctx, const float* angles_deg, int na, int w
 // Serial convention has floor(nd/2) everywhere.
 ctb_status forward_stage(ctb_ctx* ctx, const float* d_vol, int w, int h, int nz, int na, int nd,
                          const float* angles_deg, float* d_sino, float4* d_stats,
-                         cudaEvent_t* ev = nullptr, bool volume_path = false) {
+                         bool single, cudaEvent_t* ev = nullptr, bool volume_path = false) {
     const int nzg = (nz + 3) / 4;
-    const size_t elems = fwd_plane_count(nz) * std::max(fwd_plane_elems(h, w), fwd_plane_elems(w, h));
-    CTB_WS(ctx, d_img, float4, "img", elems);
-    CTB_WS(ctx, d_imgT, float4, "imgT", elems);
+    // a call's only slice has planes of 4-byte pixels of its own (a one-slice slab
+    // of a deeper stack does not: its bits are those of the whole stack's pass)
+    single = single && ctx->convention != kConvCuda;
+    const char* const img_name = single ? "img1" : "img";
+    const char* const imgT_name = single ? "imgT1" : "imgT";
+    const size_t plane = std::max(fwd_plane_elems(h, w), fwd_plane_elems(w, h));
+    const size_t elems = single ? (plane + 3) / 4 : fwd_plane_count(nz) * plane;
+    CTB_WS(ctx, d_img, float4, img_name, elems);
+    CTB_WS(ctx, d_imgT, float4, imgT_name, elems);
     CTB_WS(ctx, d_box, int4, "fbox", 2 * nzg);  // per group: box, then disc
     const int nband = (h + 7) / 8 + (w + 7) / 8;  // per group: row bands, then column bands
     CTB_WS(ctx, d_band, int2, "fband", static_cast<size_t>(nzg) * nband);
@@ -234,14 +240,15 @@ ctb_status forward_stage(ctb_ctx* ctx, const float* d_vol, int w, int h, int nz,
     // given (w, h), and normalisation writes only their interiors, so the
     // buffers' whole capacity is cleared once whenever the buffers or the plane
     // geometry change; any later group count up to the capacity reuses it
-    const size_t cap = std::min(ctx->ws["img"].bytes, ctx->ws["imgT"].bytes) / sizeof(float4);
+    const size_t cap = std::min(ctx->ws[img_name].bytes, ctx->ws[imgT_name].bytes) / sizeof(float4);
+    std::vector<long long>& zeroed = single ? ctx->img1_border_geom : ctx->img_border_geom;
     const std::vector<long long> geom = {reinterpret_cast<long long>(d_img),
                                          reinterpret_cast<long long>(d_imgT), w, h,
                                          static_cast<long long>(cap)};
-    if (ctx->img_border_geom != geom) {
+    if (zeroed != geom) {
         CTB_CUDA(ctx, cudaMemsetAsync(d_img, 0, sizeof(float4) * cap, ctx->stream));
         CTB_CUDA(ctx, cudaMemsetAsync(d_imgT, 0, sizeof(float4) * cap, ctx->stream));
-        ctx->img_border_geom = geom;
+        zeroed = geom;
     }
     Trig trig;
     CTB_TRY(trig_table(ctx, angles_deg, na, &trig));
@@ -257,14 +264,14 @@ ctb_status forward_stage(ctb_ctx* ctx, const float* d_vol, int w, int h, int nz,
         CTB_LAUNCH(ctx, launch_raymarch(d_img, w, h, nz, na, nd, det_center, trig.cs, d_sino, ctx->stream));
         return CTB_OK;
     }
-    CTB_LAUNCH(ctx, launch_normalize(d_vol, w, h, nz, d_stats, d_img, d_imgT, ctx->stream, 1, box, band));
+    CTB_LAUNCH(ctx, launch_normalize(d_vol, w, h, nz, d_stats, d_img, d_imgT, ctx->stream, 1, box, band, single));
     mark(ctx, ev, 1);
     const ctb_ctx::FwdPlanDev* plan = nullptr;
     CTB_TRY(forward_plan_dev(ctx, angles_deg, na, w, h, nd, trig, &plan));
     CTB_LAUNCH(ctx, launch_forward(d_img, d_imgT, w, h, nz, na, nd,
                                    static_cast<const int4*>(plan->groups.ptr), plan->ngroups, plan->max_strips,
                                    static_cast<const FwdAngleRec*>(plan->rec.ptr), box, band, d_sino,
-                                   ctx->stream));
+                                   ctx->stream, single));
     return CTB_OK;
 }
 
@@ -823,7 +830,7 @@ ctb_status ctb_forward_d(ctb_ctx* ctx, const float* d_vol, int n, int depth, int
     if (!aligned16(d_stats)) return fail(ctx, CTB_ERR_INVALID, "d_stats must be 16-byte aligned");
     Guard g(ctx);
     return forward_stage(ctx, d_vol, n, n, depth, num_angles, detector_bins, angles_deg, d_sino,
-                         reinterpret_cast<float4*>(d_stats));
+                         reinterpret_cast<float4*>(d_stats), depth == 1);
 }
 
 ctb_status ctb_fbp_d(ctb_ctx* ctx, const float* d_sino, int depth, int num_angles, int bins,
@@ -857,7 +864,7 @@ ctb_status ctb_reconstruct_volume_d(ctb_ctx* ctx, const float* d_vol, int n, int
     CTB_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
     mark(ctx, pev, 0);
     CTB_TRY(forward_stage(ctx, d_vol, n, n, depth, num_angles, detector_bins, nullptr, d_sino, d_stats,
-                          pev, true));
+                          depth == 1, pev, true));
     CTB_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
     mark(ctx, pev, 2);
     CTB_TRY(fbp_stage(ctx, d_sino, depth, num_angles, detector_bins, nullptr, n, filter, d_stats,
@@ -883,7 +890,7 @@ ctb_status ctb_compute_sinogram(ctb_ctx* ctx, const float* slice, int width, int
     CTB_WS(ctx, d_stats, float4, "h_stats", 1);
     CTB_CUDA(ctx, cudaMemcpyAsync(d_in, slice, npx * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     CTB_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
-    CTB_TRY(forward_stage(ctx, d_in, width, height, 1, num_angles, detector_bins, nullptr, d_sino, d_stats));
+    CTB_TRY(forward_stage(ctx, d_in, width, height, 1, num_angles, detector_bins, nullptr, d_sino, d_stats, true));
     CTB_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
     CTB_CUDA(ctx, cudaMemcpyAsync(sino_out, d_sino, ns * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     float4 st;
@@ -1021,8 +1028,8 @@ ctb_status ctb_reconstruct_volume(ctb_ctx* ctx, const float* vol, int n, int dep
         CTB_CUDA(ctx, cudaStreamWaitEvent(fwd_s, fbp_done[b], 0));  // FBP k - 2 read sino_b, stats_b
         CTB_CUDA(ctx, cudaEventRecord(t[3 * k], fwd_s));
         ctx->stream = fwd_s;
-        CTB_TRY(forward_stage(ctx, in_b, n, n, nz, num_angles, detector_bins, nullptr, sino_b, stats_b, nullptr,
-                              true));
+        CTB_TRY(forward_stage(ctx, in_b, n, n, nz, num_angles, detector_bins, nullptr, sino_b, stats_b, depth == 1,
+                              nullptr, true));
         CTB_CUDA(ctx, cudaEventRecord(fwd_done[b], fwd_s));
         if (k == ctx->fault_slab)  // test hook: fail with this slab's copy and forward stage queued
             return fail(ctx, CTB_ERR_CUDA, "injected fault after queuing slab %d of %d", k, nslab);

@@ -144,7 +144,7 @@ cudaError_t launch_slice_stats(const float* d_vol, long long npx, int nz, float4
                                int nband = 0);
 cudaError_t launch_normalize(const float* d_vol, int w, int h, int nz, const float4* d_stats,
                              float4* d_img, float4* d_imgT, cudaStream_t st, int skip_zero = 1,
-                             int4* d_box = nullptr, int2* d_band = nullptr);
+                             int4* d_box = nullptr, int2* d_band = nullptr, bool single = false);
 // The reference CUDA backend's ray-march forward projector over the
 // normalised image planes (img only).
 cudaError_t launch_raymarch(const float4* d_img, int w, int h, int nz, int na, int nd, float det_center,
@@ -203,7 +203,7 @@ cudaError_t launch_fwd_angles(const int4* d_groups, int ngroups, const int* d_or
 cudaError_t launch_forward(const float4* d_img, const float4* d_imgT, int w, int h, int nz,
                            int na, int nd, const int4* d_groups, int ngroups, int max_strips,
                            const FwdAngleRec* d_rec, const int4* d_box, const int2* d_band, float* d_sino,
-                           cudaStream_t st);
+                           cudaStream_t st, bool single = false);
 // Twiddle tables of the filter's FFT of length L (every radix-16 pass and the
 // radix-2/4/8 last pass, r-major per pass), correctly rounded from double
 // precision: fft_twiddle_len(L) float2 entries; for L <= kPackedMaxL followed,
@@ -370,7 +370,8 @@ struct ctb_ctx {
         int ngroups = 0, max_strips = 0;
     };
     std::map<std::vector<long long>, FwdPlanDev> fwd_plans;
-    std::vector<long long> img_border_geom;  // geometry the image borders were zeroed for
+    // geometry the image borders were zeroed for: stacks, single slices
+    std::vector<long long> img_border_geom, img1_border_geom;
     unsigned* d_err = nullptr;  // device error word for bounded waits
     int fault_slab = -1;        // host-side fault injection in the volume pipeline (tests)
 

@@ -152,12 +152,13 @@ __global__ void __launch_bounds__(1024) k_slice_stats(const float* __restrict__ 
 // only where its intervals meet that box and that disc, every other pixel
 // being an exact zero. With band set, the group's ceil(h/8) row bands (8 rows
 // each) get the x range of their non-zero pixels, followed by its ceil(w/8)
-// column bands with their y range (emptied by k_slice_stats too).
+// column bands with their y range (emptied by k_slice_stats too). With single, the
+// copies of a one-slice stack are planes of 4-byte pixels in the same layout.
 __global__ void __launch_bounds__(256) k_normalize(const float* __restrict__ vol, int w, int h, int nz,
                                                    const float4* __restrict__ stats,
                                                    float4* __restrict__ img, float4* __restrict__ imgT,
                                                    int skip_zero, int4* __restrict__ box,
-                                                   int2* __restrict__ band) {
+                                                   int2* __restrict__ band, int single) {
     const long long pw = w + 2 * kFwdGuard, ph = h + 2 * kFwdGuard;  // row pitches
     const long long rw = h + kFwdRows, rh = w + kFwdRows;             // rows per plane
     __shared__ float4 tile[32][33];
@@ -205,7 +206,10 @@ __global__ void __launch_bounds__(256) k_normalize(const float* __restrict__ vol
             r4 = max(r4, dx * dx + dy * dy);
         }
         tile[ty + 8 * r][tx] = q;
-        if (x < w && y < h) img[((zg / 2 * rw + y) * pw + x + kFwdGuard) * 2 + (zg & 1)] = q;
+        if (x < w && y < h) {
+            if (single) reinterpret_cast<float*>(img)[y * pw + x + kFwdGuard] = q.x;
+            else img[((zg / 2 * rw + y) * pw + x + kFwdGuard) * 2 + (zg & 1)] = q;
+        }
     }
     __shared__ int4 wbox[8];  // per warp, then one set of atomics per block
     __shared__ int wr4[8];
@@ -281,7 +285,10 @@ __global__ void __launch_bounds__(256) k_normalize(const float* __restrict__ vol
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int x = x0 + ty + 8 * r, y = y0 + tx;
-        if (imgT && x < w && y < h) imgT[((zg / 2 * rh + x) * ph + y + kFwdGuard) * 2 + (zg & 1)] = tile[tx][ty + 8 * r];
+        if (imgT && x < w && y < h) {
+            if (single) reinterpret_cast<float*>(imgT)[x * ph + y + kFwdGuard] = tile[tx][ty + 8 * r].x;
+            else imgT[((zg / 2 * rh + x) * ph + y + kFwdGuard) * 2 + (zg & 1)] = tile[tx][ty + 8 * r];
+        }
     }
 }
 
@@ -383,10 +390,10 @@ cudaError_t launch_slice_stats(const float* d_vol, long long npx, int nz, float4
 
 cudaError_t launch_normalize(const float* d_vol, int w, int h, int nz, const float4* d_stats,
                              float4* d_img, float4* d_imgT, cudaStream_t st, int skip_zero,
-                             int4* d_box, int2* d_band) {
+                             int4* d_box, int2* d_band, bool single) {
     const dim3 grid(2 * ((w + 31) / 32), (h + 31) / 32, (nz + 7) / 8);
     return launch_chained(k_normalize, grid, 256, 0, st, d_vol, w, h, nz, d_stats, d_img, d_imgT, skip_zero, d_box,
-                          d_band);
+                          d_band, single ? 1 : 0);
 }
 
 }  // namespace ctb

@@ -129,6 +129,20 @@ __device__ __forceinline__ void walk_rows(const float4* __restrict__ lane_base, 
     }
 }
 
+// The same for a single slice (4-byte pixels), two rows at a time: the two lanes
+// of a packed operation hold an even and an odd row, so the weights need no copies.
+__device__ __forceinline__ void walk_rows(const float* __restrict__ lane_base, const RowRec* __restrict__ rr, float cl1,
+                                          float2 (&acc)[3]) {
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+        const float2 v = make_float2(__ldg(lane_base + rr[i].col), __ldg(lane_base + rr[i + 1].col));
+        const float2 y = make_float2(cl1 + rr[i].dy, cl1 + rr[i + 1].dy);
+        acc[0] = __ffma2_rn(make_float2(fmaxf(-y.x, 0.0f), fmaxf(-y.y, 0.0f)), v, acc[0]);
+        acc[1] = __ffma2_rn(make_float2(1.0f - fabsf(y.x), 1.0f - fabsf(y.y)), v, acc[1]);
+        acc[2] = __ffma2_rn(make_float2(fmaxf(y.x, 0.0f), fmaxf(y.y, 0.0f)), v, acc[2]);
+    }
+}
+
 // Bins 0 and nd-1 by the reference's rules (SerialBackend.cpp:109-120), on
 // its own float s: bin 0 takes (1 - frac) v from the pixels with floor(s) =
 // 0, bin nd-1 takes frac v from floor(s) = nd-2 and v from floor(s) = nd-1.
@@ -179,6 +193,43 @@ __device__ __noinline__ void edge_bin(const float4* __restrict__ plane, int pitc
         }
 }
 
+// edge_bin of a single slice.
+__device__ __noinline__ float edge_bin(const float* __restrict__ plane, int pitch, int nq, const FAngle& f, int b_lo, int e,
+                                       int nd, int r_lo, int r_hi, bool rows, float cxf, float cyf, int lane) {
+    float sum = 0.0f;
+    const double lo = e == 0 ? 0.0 : nd - 2.0, hi = e == 0 ? 1.0 : static_cast<double>(nd);
+    const double da = (lo - 1.0 / 64 - b_lo) * f.inv, db = (hi + 1.0 / 64 - b_lo) * f.inv;
+    const float dcs = static_cast<float>(nd / 2);
+    for (int p = r_lo + lane; p <= r_hi; p += LANES) {
+        const double qp = fma(static_cast<double>(p), f.dq, f.q0);
+        const int c0 = static_cast<int>(ceil(qp + fmin(da, db)));
+        const int c1 = min(static_cast<int>(floor(qp + fmax(da, db))), nq - 1);
+        // at most (2 + 1/32) sqrt(2) < 3 columns; the loads do not wait for the weights
+        float wgt[3], v[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int c = c0 + i;
+            const bool in = c >= 0 && c <= c1;
+            v[i] = __ldg(plane + static_cast<long long>(p) * pitch + (in ? c : 0));
+            const float xg = static_cast<float>(rows ? c : p);
+            const float yg = static_cast<float>(rows ? p : c);
+            const float ss = __fadd_rn(__fadd_rn(__fmul_rn(__fsub_rn(xg, cxf), f.cf),
+                                                 __fmul_rn(__fsub_rn(yg, cyf), f.sf)), dcs);
+            const float fl = floorf(ss);
+            const int i0 = static_cast<int>(fl);
+            const float fr = __fsub_rn(ss, fl);
+            if (e == 0) wgt[i] = i0 == 0 ? __fsub_rn(1.0f, fr) : 0.0f;
+            else wgt[i] = i0 == nd - 2 ? fr : (i0 == nd - 1 ? 1.0f : 0.0f);
+            if (!in) wgt[i] = 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            if (wgt[i] != 0.0f) sum = fmaf(wgt[i], v[i], sum);
+    }
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    return sum;
+}
+
 // PER_SM: the CTAs per SM the registers are held to. Seven (72 registers) for
 // launches that fill the SMs. A launch that does not is bound by the latency of its
 // loads: four per SM (127 registers) let a warp have all eight rows of a group on
@@ -186,7 +237,11 @@ __device__ __noinline__ void edge_bin(const float4* __restrict__ plane, int pitc
 // 180, 39.0 and 29.8 at 128^2 x 8 x 180, 28.7 and 22.6 at 64^2 x 1 x 90; but 72.0
 // and 73.3 at 256^2 x 1 x 360 with 1620 CTAs, 2563 and 2714 at 512^2 x 64 x 720).
 constexpr int FULL = 7, SPARSE = 4;
-template <int PER_SM>
+// ONE: a single slice in planes of 4-byte pixels (img, imgT then point to floats):
+// a row of 32 columns is one or two L1 wavefronts instead of nine and a row takes a
+// quarter of the instructions (us of a whole call: 27.3 -> 18.8 at 160^2 x 180, 66.5 ->
+// 34.6 at 256^2 x 360, 348 -> 154 at 512^2 x 720, 2336 -> 991 at 1024^2 x 1440).
+template <int PER_SM, bool ONE>
 __global__ void __launch_bounds__(THREADS, PER_SM)
     k_forward(const float4* __restrict__ img, const float4* __restrict__ imgT, int w, int h, int nz, int na, int nd,
               const int4* __restrict__ groups, const FwdAngleRec* __restrict__ arec, const int4* __restrict__ box,
@@ -328,11 +383,12 @@ __global__ void __launch_bounds__(THREADS, PER_SM)
     const int nby = (h + 7) / 8, nbx = (w + 7) / 8;
     const int nb_all = nby + nbx, nb_off = rows ? 0 : nby, nb_p = rows ? nby : nbx;
 
-    float2 acc[3][2 * NP];
+    float2 acc[3][ONE ? 1 : 2 * NP];
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int j = 0; j < 2 * NP; ++j) acc[r][j] = make_float2(0.0f, 0.0f);
+        for (int j = 0; j < (ONE ? 1 : 2 * NP); ++j) acc[r][j] = make_float2(0.0f, 0.0f);
+    const float* plane1 = reinterpret_cast<const float*>(rows ? img : imgT) + kFwdGuard;  // of a single slice
     if (has_a) {
         const FAngle& f = fa[ja];
         const float akq = f.akq;
@@ -374,8 +430,18 @@ __global__ void __launch_bounds__(THREADS, PER_SM)
                 plane + 2 * (static_cast<long long>(p0) * pitch - kFwdGuard + (f.neg ? -lane : lane));
             // groups of 8 rows without a needed one add only zeros
 #pragma unroll 1
-            for (int g = 0; g < LANES; g += 8)
-                if ((need >> g) & 0xffu) walk_rows(lane_base, rr + g, cl1, acc);
+            for (int g = 0; g < LANES; g += 8) {
+                if (!((need >> g) & 0xffu)) continue;
+                if constexpr (ONE) {
+                    float2 a[3] = {acc[0][0], acc[1][0], acc[2][0]};
+                    walk_rows(plane1 + (static_cast<long long>(p0) * pitch - kFwdGuard + (f.neg ? -lane : lane)), rr + g,
+                              cl1, a);
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) acc[r][0] = a[r];
+                } else {
+                    walk_rows(lane_base, rr + g, cl1, acc);
+                }
+            }
         }
     }
     if (!has_a) return;
@@ -393,9 +459,12 @@ __global__ void __launch_bounds__(THREADS, PER_SM)
     const int mprev = __shfl_up_sync(kAll, ml, 1);
     const unsigned firsts = __ballot_sync(kAll, lane == 0 || mprev != ml);
     const int t = lane + 1;
-    float2 sum[2 * NP];
+    constexpr int NS = ONE ? 1 : 2 * NP;
+    if constexpr (ONE)  // the even and the odd rows
+        for (int r = 0; r < 3; ++r) acc[r][0] = make_float2(acc[r][0].x + acc[r][0].y, 0.0f);
+    float2 sum[NS];
 #pragma unroll
-    for (int j = 0; j < 2 * NP; ++j) sum[j] = make_float2(0.0f, 0.0f);
+    for (int j = 0; j < NS; ++j) sum[j] = make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int r = 2; r >= 0; --r) {
         const unsigned l0 = __fns(firsts, 0, t - r + 2);  // first lane of run t - r (or ~0u: none)
@@ -403,9 +472,11 @@ __global__ void __launch_bounds__(THREADS, PER_SM)
         const bool ok1 = ok0 && l0 + 1 < LANES && !((firsts >> (l0 + 1)) & 1u);
         const int s0 = ok0 ? static_cast<int>(l0) : lane, s1 = ok1 ? static_cast<int>(l0) + 1 : lane;
 #pragma unroll
-        for (int j = 0; j < 2 * NP; ++j) {
-            const float2 a0 = make_float2(__shfl_sync(kAll, acc[r][j].x, s0), __shfl_sync(kAll, acc[r][j].y, s0));
-            const float2 a1 = make_float2(__shfl_sync(kAll, acc[r][j].x, s1), __shfl_sync(kAll, acc[r][j].y, s1));
+        for (int j = 0; j < NS; ++j) {
+            const float2 a0 = make_float2(__shfl_sync(kAll, acc[r][j].x, s0),
+                                          ONE ? 0.0f : __shfl_sync(kAll, acc[r][j].y, s0));
+            const float2 a1 = make_float2(__shfl_sync(kAll, acc[r][j].x, s1),
+                                          ONE ? 0.0f : __shfl_sync(kAll, acc[r][j].y, s1));
             if (ok0) sum[j] = __fadd2_rn(sum[j], a0);
             if (ok1) sum[j] = __fadd2_rn(sum[j], a1);
         }
@@ -413,10 +484,10 @@ __global__ void __launch_bounds__(THREADS, PER_SM)
     const int b = b_lo + t;
     if (lane < nout && b != 0 && b != nd - 1) {
 #pragma unroll
-        for (int j = 0; j < 2 * NP; ++j) {
+        for (int j = 0; j < NS; ++j) {
             const int z = 4 * g0 + 2 * j;  // slices z, z + 1 of pair j
             if (z < nz) sino[z * zst + ob + b] = sum[j].x;
-            if (z + 1 < nz) sino[(z + 1) * zst + ob + b] = sum[j].y;
+            if (!ONE && z + 1 < nz) sino[(z + 1) * zst + ob + b] = sum[j].y;
         }
     }
     // bins 0 and nd-1 on the reference's own rules
@@ -424,6 +495,12 @@ __global__ void __launch_bounds__(THREADS, PER_SM)
     for (int side = 0; side < 2; ++side) {
         if (!(side == 0 ? has0 : has_last)) continue;
         const int eb = side == 0 ? 0 : nd - 1;
+        if constexpr (ONE) {
+            const float v = edge_bin(plane1, pitch, nq, f, b_lo, eb, nd, erow[ja][2 * side], erow[ja][2 * side + 1], rows,
+                                     cxf, cyf, lane);
+            if (lane == 0) sino[ob + eb] = v;
+            continue;
+        }
         float2 sum[2 * NP];
         edge_bin(plane, pitch, nq, f, b_lo, eb, nd, erow[ja][2 * side], erow[ja][2 * side + 1], rows, cxf,
                  cyf, lane, sum);
@@ -469,13 +546,15 @@ __global__ void k_fwd_angles(const int4* __restrict__ groups, int ngroups, const
 cudaError_t launch_forward(const float4* d_img, const float4* d_imgT, int w, int h, int nz,
                            int na, int nd, const int4* d_groups, int ngroups, int max_strips,
                            const FwdAngleRec* d_rec, const int4* d_box, const int2* d_band, float* d_sino,
-                           cudaStream_t st) {
+                           cudaStream_t st, bool single) {
     const dim3 grid(max_strips, ngroups, ((nz + 3) / 4 + NP - 1) / NP);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const bool sparse = static_cast<long long>(grid.x) * grid.y * grid.z <= static_cast<long long>(SPARSE) * sms;
-    return launch_chained(sparse ? k_forward<SPARSE> : k_forward<FULL>, grid, dim3(LANES, GMAX), 0, st, d_img, d_imgT, w,
+    auto kernel = single ? (sparse ? k_forward<SPARSE, true> : k_forward<FULL, true>)
+                         : (sparse ? k_forward<SPARSE, false> : k_forward<FULL, false>);
+    return launch_chained(kernel, grid, dim3(LANES, GMAX), 0, st, d_img, d_imgT, w,
                           h, nz, na, nd, d_groups, d_rec, d_box, d_band, d_sino);
 }
 

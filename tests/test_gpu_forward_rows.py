@@ -46,3 +46,22 @@ def test_rows_meet_parity(backend, region, n, depth, bounds):
         ref = O.sinogram_f64(vol[z], na, nd, ang)[0]
         assert np.all(np.isfinite(got[z]))
         assert np.linalg.norm(got[z] - ref) <= 1e-5 * max(np.linalg.norm(ref), 1e-30) + 1e-12
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (5, 40), (64, 33), (97, 70)])
+@pytest.mark.parametrize("nd_of", ["width", "two", "wide"])
+def test_single_slice_meets_parity(backend, w, h, nd_of):
+    """A call's only slice has planes and a walk of its own: rectangular images,
+    detectors that cut the image and that reach past it, and a call of another
+    size in between (the planes' zero borders)."""
+    rng = np.random.default_rng(w * h)
+    img = rng.uniform(-1.0, 1.0, (h, w)).astype(np.float32)
+    img[rng.uniform(size=(h, w)) < 0.3] = 0.0
+    nd = {"width": max(w, 2), "two": 2, "wide": 2 * max(w, h) + 3}[nd_of]
+    na = 31
+    first = backend.computeSinogram(img, na, nd)
+    backend.computeSinogram(np.ones((h + 3, w + 2), np.float32), na, nd + 1)
+    again = backend.computeSinogram(img, na, nd)
+    np.testing.assert_array_equal(first.data, again.data)
+    ref = O.sinogram_f32(img, na, nd)[0]
+    assert np.linalg.norm(first.data - ref) <= 1e-5 * max(np.linalg.norm(ref), 1e-30) + 1e-12
