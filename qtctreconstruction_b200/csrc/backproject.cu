@@ -69,12 +69,16 @@ constexpr int THREADS = 256;
 constexpr float kRound = 12582912.0f;   // 1.5 * 2^23: x + kRound rounds x to an integer
 constexpr int kRoundBits = 0x4B400000;  // bit pattern of kRound
 
-// A tile shape: TX x TY voxels in columns of V, a ring of NST stages of CA / 2
-// windows (one per angle and slice group) and WIN bins per window: with a span of
-// sqrt((TX-1)^2 + (TY-1)^2) bins, the taps of every column lie in bins 0 ..
-// floor(span + 2) + 2 of the window. MINB is the launch-bounds occupancy target (registers 65536 / (256 MINB)).
+// A tile shape: TX x TY voxels in columns of V, a ring of NST stages of SW windows
+// (one per angle and slice group; about 2 CA in all) and WIN bins per window: with
+// a span of sqrt((TX-1)^2 + (TY-1)^2) bins, the taps of every column lie in bins 0
+// .. floor(span + 2) + 2 of the window. MINB is the launch-bounds occupancy target
+// (registers 65536 / (256 MINB)). A stage costs every warp about 80 instructions
+// beside its angles, so few large stages beat many small ones as long as three CTAs
+// fit an SM (32x32 tile at 512^2 x 256 x 720: 5.58 ms with 5 stages of 16 windows,
+// 5.75 with 6 of 12, 5.51 with 4 of 20, 5.28 with 3 of 26).
 constexpr int V = 4;
-template <int TX_, int TY_, int CA_, int WIN_, int NST_, int MINB_, bool PAIR_>
+template <int TX_, int TY_, int CA_, int WIN_, int SW_, int NST_, int MINB_, bool PAIR_>
 struct Shape {
     static constexpr int TX = TX_, TY = TY_, CA = CA_, WIN = WIN_, MINB = MINB_;
     static constexpr bool PAIR = PAIR_;
@@ -83,7 +87,7 @@ struct Shape {
     // the last stage's slot made every producer wait for the slowest warp: 13.3
     // against 11.4 ms at 512^3 x 720).
     static constexpr int NST = NST_, AHEAD = NST - 2;
-    static constexpr int SW = CA / 2;                                // windows per stage
+    static constexpr int SW = SW_;                                   // windows per stage
     static constexpr int COLS = TX * TY / V;                         // columns of a tile
     static constexpr int SPLIT = COLS >= THREADS ? 1 : THREADS / COLS;  // groups that share a chunk's angles
     static constexpr int GT = THREADS / SPLIT;                       // threads per group
@@ -95,12 +99,12 @@ struct Shape {
     static_assert(WIN <= kBpWindowMax, "window within the filtered-row guard");
     static_assert(SPLIT * V * GT <= SPLIT * TX * TY, "the exchange buffer holds every group's sums");
 };
-using V0 = Shape<32, 32, 32, 48, 5, 3, true>;  // the general-purpose shape
-using V1 = Shape<64, 32, 32, 76, 4, 2, false>;  // wide tiles: less staging per voxel
-using V2 = Shape<32, 16, 32, 40, 5, 3, true>;  // half-height tiles: twice the CTAs
-using V3 = Shape<16, 16, 32, 28, 5, 3, true>;  // small tiles for small slices
-using V4 = Shape<32, 32, 16, 48, 5, 3, true>;  // the general shape with half the ring
-using V5 = Shape<32, 32, 64, 48, 4, 2, true>;  // the general shape with twice the ring (half the stages)
+using V0 = Shape<32, 32, 32, 48, 26, 3, 3, true>;  // the general-purpose shape
+using V1 = Shape<64, 32, 32, 76, 16, 4, 2, false>;  // wide tiles: less staging per voxel
+using V2 = Shape<32, 16, 32, 40, 24, 4, 3, true>;  // half-height tiles: twice the CTAs
+using V3 = Shape<16, 16, 32, 28, 24, 4, 3, true>;  // small tiles for small slices
+using V4 = Shape<32, 32, 16, 48, 12, 3, 3, true>;  // the general shape with half the ring
+using V5 = Shape<32, 32, 64, 48, 32, 4, 2, true>;  // the general shape with twice the ring (half the stages)
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
     return static_cast<unsigned>(__cvta_generic_to_shared(p));
