@@ -279,8 +279,11 @@ __global__ void __launch_bounds__(THREADS, PER_SM)
         if (dq != 0.0) {
             const double pa0 = (cl - kReach - qa) * idq, pb0 = (ch + kReach - qa) * idq;
             const double pa1 = (cl - kReach - qb) * idq, pb1 = (ch + kReach - qb) * idq;
-            lo = max(rl, static_cast<int>(floor(fmin(fmin(pa0, pb0), fmin(pa1, pb1)))) - 1);
-            hi = min(rh, static_cast<int>(ceil(fmax(fmax(pa0, pb0), fmax(pa1, pb1)))) + 1);
+            // clamped to [rl, rh + 1] and [rl - 1, rh] before the conversion: at an
+            // angle one float step off an axis (90 degrees of 670 uniform ones) idq
+            // is 7.5e6, and the rows of columns 286 away do not fit an int
+            lo = static_cast<int>(fmin(fmax(floor(fmin(fmin(pa0, pb0), fmin(pa1, pb1))) - 1.0, rl), rh + 1.0));
+            hi = static_cast<int>(fmax(fmin(ceil(fmax(fmax(pa0, pb0), fmax(pa1, pb1))) + 1.0, rh), rl - 1.0));
         } else if (fmax(qa, qb) < cl - kReach || fmin(qa, qb) > ch + kReach) {
             hi = -1;
         }

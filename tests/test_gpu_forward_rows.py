@@ -65,3 +65,28 @@ def test_single_slice_meets_parity(backend, w, h, nd_of):
     np.testing.assert_array_equal(first.data, again.data)
     ref = O.sinogram_f32(img, na, nd)[0]
     assert np.linalg.norm(first.data - ref) <= 1e-5 * max(np.linalg.norm(ref), 1e-30) + 1e-12
+
+
+@pytest.mark.parametrize("nd", [640, 1283])
+@pytest.mark.parametrize("depth", [1, 3])
+def test_angles_next_to_an_axis(backend, depth, nd):
+    """Angles a float step (and much less) away from an axis: the rows where a strip
+    meets a column far away do not fit an int. At an even n and these angles s lies
+    half way between bins, so the float rules of the outer bins are not at an edge."""
+    import torch
+    n = 640
+    rng = np.random.default_rng(depth)
+    vol = rng.uniform(0.5, 1.5, (depth, n, n)).astype(np.float32)
+    near = np.float32(90.0)
+    ang = np.array([np.nextafter(near, np.float32(0)), near, np.nextafter(near, np.float32(180)), 1e-30, 1e-5,
+                    np.nextafter(np.float32(180), np.float32(0)), 37.0], np.float32)
+    d_v = torch.from_numpy(vol).cuda()
+    d_s = torch.full((depth, len(ang), nd), float("nan"), device="cuda")
+    d_st = torch.empty(depth, 4, device="cuda")
+    backend.forward_d(d_v.data_ptr(), n, depth, len(ang), nd, d_s.data_ptr(), d_st.data_ptr(), ang)
+    backend.synchronize()
+    got = d_s.cpu().numpy()
+    for z in range(depth):
+        ref = O.sinogram_f64(vol[z], len(ang), nd, ang)[0]
+        for k in range(len(ang)):
+            assert np.linalg.norm(got[z, k] - ref[k]) <= 1e-5 * np.linalg.norm(ref[k]), (z, ang[k])
