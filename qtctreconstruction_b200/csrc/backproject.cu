@@ -34,13 +34,13 @@
 // once, and lanes next to each other read bins next to each other, without bank
 // conflicts. Each voxel adds three taps with hat weights; which three depends on
 // the slow coefficient alone (four patterns, column_taps), and two slice groups
-// share the weights. The kernel is then bound by issue: 48 packed FP32x2
-// operations of two issue cycles and about 62 other instructions per column and
-// angle of 8 slices (11.03 ms at 512^3 x 720; FMA pipe 67 %, shared memory 75 %
-// busy; with two of the taps read only, 10.95 ms). Measured and not kept: tap
-// differences with saturating weights, which share the first tap's sum within a
-// column (11.72 ms), one slice group per item (13.4 ms) or four (11.07 ms), 64 or
-// 128 registers (12.4 and 11.3 ms against 80).
+// share the weights. The kernel is then bound by issue: 48 packed FP32x2 FMAs of
+// two issue cycles (6.8 ms on their own) and about 40 other instructions per column
+// and angle of 8 slices: 10.46 ms at 512^3 x 720, FMA pipe 69 %, shared memory 78 %
+// busy (11.03 ms with smaller stages, see Shape). Measured then, against 11.03: with
+// two of the taps read only, 10.95 ms; not kept: tap differences with saturating
+// weights, which share the first tap's sum within a column (11.72), one slice group
+// per item (13.4) or four (11.07), 64 or 128 registers (12.4 and 11.3 against 80).
 //
 // The slow axis is x for angles with |sin| > |cos| and y for the others, so a
 // tile runs through the angles in the order of the table (Trig): first those
@@ -668,9 +668,28 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
     }
 }
 
+// Dynamic shared memory of a launch with one CTA per item. Tiles outside the
+// circle end at once, and CTAs are handed out before that is known: with 1.9 items
+// of work per SM some SMs get three and others one. Where those items need fewer
+// CTAs per SM than fit (b.per_sm), a CTA therefore asks for so much shared memory
+// that no more than those fit, and the rest go to the SMs that come free. Measured,
+// FBP: 330 -> 235 us at 387^2 x 16 x 580, 200 -> 143 at 387^2 x 8, 50.4 -> 42.1 at
+// 200^2 x 8 x 314 in 16x16 tiles. Not where all CTAs are resident that way anyhow
+// (b.per_sm = 0), which only costs: 27.8 -> 31.7 at 96^2 x 24 x 150.
+constexpr int kSmemPerSm = 228 * 1024, kSmemPerCta = 1024;  // of an SM; what each CTA takes besides
+constexpr int smem_for(int own, int per_sm) {
+    const int floor = kSmemPerSm / (per_sm + 1) - kSmemPerCta + 128;  // per_sm + 1 CTAs do not fit
+    return own > floor ? own : floor;
+}
+template <class C>
+size_t item_smem(const BpBatch& b) {
+    const int own = static_cast<int>(sizeof(BpSmem<C>));
+    return static_cast<size_t>(b.per_sm >= 1 && b.per_sm < C::MINB ? smem_for(own, b.per_sm) : own);
+}
+
 template <class C>
 cudaError_t set_smem() {
-    const int bytes = static_cast<int>(sizeof(BpSmem<C>));
+    const int bytes = smem_for(static_cast<int>(sizeof(BpSmem<C>)), 1);
     cudaError_t e = cudaFuncSetAttribute(k_backproject<C, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_backproject<C, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -688,7 +707,7 @@ template <class C>
 cudaError_t launch_one(const BpBatch& b, unsigned* d_err, cudaStream_t st) {
     cudaError_t e = set_smem<C>();
     if (e != cudaSuccess) return e;
-    k_backproject<C, 0><<<static_cast<unsigned>(b.total), THREADS, sizeof(BpSmem<C>), st>>>(b, nullptr, d_err);
+    k_backproject<C, 0><<<static_cast<unsigned>(b.total), THREADS, item_smem<C>(b), st>>>(b, nullptr, d_err);
     return cudaGetLastError();
 }
 
@@ -697,7 +716,7 @@ cudaError_t launch_many(const BpBatch& b, bool persistent, unsigned* d_counter, 
     cudaError_t e = set_smem<C>();
     if (e != cudaSuccess) return e;
     if (!persistent) {
-        k_backproject<C, 1><<<static_cast<unsigned>(b.total), THREADS, sizeof(BpSmem<C>), st>>>(b, nullptr, d_err);
+        k_backproject<C, 1><<<static_cast<unsigned>(b.total), THREADS, item_smem<C>(b), st>>>(b, nullptr, d_err);
         return cudaGetLastError();
     }
     int dev = 0, sms = 0, per_sm = 0;
@@ -758,7 +777,7 @@ long long active_tiles(int n, const BpShape& sh, double ctr) {
 // (its 8 warps do not fill it); beyond it the SMs even out to half an item.
 // Costs per item (one or
 // two slice groups) relative to a 32x32 tile of one group, from the
-// backprojector's time at 512^2 x 64 x 720: 32x32 1.658 and 1.462 ms, 32x16
+// backprojector's time at 512^2 x 64 x 720 (with stages of 16 windows): 32x32 1.658 and 1.462 ms, 32x16
 // 1.822 and 1.640 ms, 16x16 2.173 and 2.082 ms.
 double launch_cost(int variant, int zgs, long long items, int sms) {
     const double pair = variant == 2 ? 0.99 : variant == 3 ? 0.63 : 1.76;
@@ -778,11 +797,10 @@ long long active_items(const BpJob& J, int variant, int zgs) {
 int bp_default_variant(int n_out, int nz, int sms) {
     // The shape whose launch is estimated fastest for the job alone; a smaller
     // tile has to gain 15 % in the estimate, which leaves its own start-up cost
-    // out. Measured on B200, us, 32x32 / 32x16 / 16x16: 24.0 for 16x16
-    // at 64^2 x 16 x 101 (30.2 for 32x32); 40.4 / 38.3 / 50.6 at 128^2 x 32 x
-    // 201; 187.8 / 144.7 / 157.1 at 387^2 x 8 x 580; 1462 / 1640 / 2082 at 512^2
-    // x 64 x 720. The 64x32 tile and the other chunk sizes are left to the
-    // autotuner.
+    // out. Measured on B200, us per FBP, 32x32 / 32x16 / 16x16: 27.8 / 21.7 / 19.7
+    // at 64^2 x 16 x 101; 46.2 / 44.1 / 54.3 at 128^2 x 32 x 201; 142.6 / 141.0 /
+    // 161.6 at 387^2 x 8 x 580; 1565 / 1714 / 1991 at 512^2 x 64 x 720. The 64x32
+    // tile and the other rings are left to the autotuner.
     BpJob J;
     J.n = n_out;
     J.nz = nz;
@@ -818,6 +836,8 @@ void bp_number_items(BpBatch& b, int variant, int sms) {
         J.first = b.total;
         b.total += static_cast<long long>(J.tiles) * (((J.nz + 3) / 4 + J.zgs - 1) / J.zgs);
     }
+    const long long active = pair ? two : one, per_sm = (active + sms - 1) / sms;
+    b.per_sm = per_sm < 16 && b.total > per_sm * sms ? static_cast<int>(per_sm) : 0;
 }
 
 FiltLayout filt_layout(int sq, int n_out) {

@@ -266,6 +266,7 @@ struct BpJob {
 };
 struct BpBatch {
     int njobs = 0;
+    int per_sm = 0;  // most CTAs per SM that balance the items with work, 0: any (bp_number_items)
     long long total = 0;
     BpJob job[kMaxJobs];
 };

@@ -68,3 +68,20 @@ def test_slice_pairs_do_not_change_bits(backend, depth, shape):
     deep = _fbp(backend, np.concatenate([sinos[:4]] * 8 + [sinos]), ang, n, shape)[32:]
     for z in range(0, depth, 4):
         np.testing.assert_array_equal(deep[z:min(z + 4, depth)], _fbp(backend, sinos[z:z + 4], ang, n, shape))
+
+
+@pytest.mark.parametrize("shape", [0, 2, 3])
+@pytest.mark.parametrize("n,depth", [(387, 1), (387, 8), (387, 16), (200, 8)])
+def test_fewer_ctas_per_sm_than_fit(backend, n, depth, shape):
+    """Launches whose tiles inside the circle need one or two CTAs per SM while there
+    are more tiles than that: every tile, inside or outside, is still written."""
+    na, bins = 7, ctb.odd_detector_count(n)
+    rng = np.random.default_rng(n + depth)
+    sinos = rng.uniform(0.0, 1.0, (depth, na, bins)).astype(np.float32)
+    ang = O.uniform_angles_deg(na)
+    got = _fbp(backend, sinos, ang, n, shape)
+    assert np.all(np.isfinite(got))
+    for z in {0, depth - 1}:
+        ref = O.reconstruct_slice_f64(sinos[z], ang, n, int(FilterType.SheppLogan))
+        assert O.rel_l2(got[z], ref) <= 1e-5
+        assert O.max_abs_rel(got[z], ref) <= 1e-4
