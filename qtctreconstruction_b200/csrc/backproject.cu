@@ -34,8 +34,8 @@
 // once, and lanes next to each other read bins next to each other, without bank
 // conflicts. Each voxel adds three taps with hat weights; which three depends on
 // the slow coefficient alone (four patterns, column_taps), and two slice groups
-// share the weights. The kernel is then bound by issue: 48 packed FP32x2 FMAs of
-// two issue cycles (6.8 ms on their own) and about 40 other instructions per column
+// share the weights. The kernel is then bound by issue: 44 packed FP32x2 FMAs of
+// two issue cycles (6.2 ms on their own) and about 43 other instructions per column
 // and angle of 8 slices: 10.46 ms at 512^3 x 720, FMA pipe 69 %, shared memory 78 %
 // busy (11.03 ms with smaller stages, see Shape). Measured then, against 11.03: with
 // two of the taps read only, 10.95 ms; not kept: tap differences with saturating
@@ -775,10 +775,9 @@ long long active_tiles(int n, const BpShape& sh, double ctr) {
 // an SM times an item's cost. Three items fit an SM at once: up to that count
 // the fullest SM decides, a lone item taking 1.4 times its share of a full SM
 // (its 8 warps do not fill it); beyond it the SMs even out to half an item.
-// Costs per item (one or
-// two slice groups) relative to a 32x32 tile of one group, from the
-// backprojector's time at 512^2 x 64 x 720 (with stages of 16 windows): 32x32 1.658 and 1.462 ms, 32x16
-// 1.822 and 1.640 ms, 16x16 2.173 and 2.082 ms.
+// Costs per item (one or two slice groups) relative to a 32x32 tile of one group,
+// from the backprojector's time at 512^2 x 64 x 720 (with stages of 16 windows):
+// 32x32 1.658 and 1.462 ms, 32x16 1.822 and 1.640, 16x16 2.173 and 2.082.
 double launch_cost(int variant, int zgs, long long items, int sms) {
     const double pair = variant == 2 ? 0.99 : variant == 3 ? 0.63 : 1.76;
     const double one = variant == 2 ? 0.55 : variant == 3 ? 0.33 : 1.0;
