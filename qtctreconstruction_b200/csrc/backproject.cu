@@ -668,28 +668,29 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
     }
 }
 
-// Dynamic shared memory of a launch with one CTA per item. Tiles outside the
-// circle end at once, and CTAs are handed out before that is known: with 1.9 items
-// of work per SM some SMs get three and others one. Where those items need fewer
-// CTAs per SM than fit (b.per_sm), a CTA therefore asks for so much shared memory
-// that no more than those fit, and the rest go to the SMs that come free. Measured,
-// FBP: 330 -> 235 us at 387^2 x 16 x 580, 200 -> 143 at 387^2 x 8, 50.4 -> 42.1 at
-// 200^2 x 8 x 314 in 16x16 tiles. Not where all CTAs are resident that way anyhow
-// (b.per_sm = 0), which only costs: 27.8 -> 31.7 at 96^2 x 24 x 150.
+// Launches with one CTA per item whose items with work need fewer CTAs per SM
+// (b.per_sm) than fit: a CTA asks for so much shared memory that no more than those
+// fit. Tiles outside the circle end at once, and CTAs are handed out before that is
+// known: with 1.9 items of work per SM some SMs got three and others one; now the rest
+// go to the SMs that come free. Measured, FBP: 330 -> 235 us at 387^2 x 16 x 580, 200
+// -> 143 at 387^2 x 8, 50.4 -> 42.1 at 200^2 x 8 x 314 in 16x16 tiles.
+// Where every CTA is resident anyhow (not b.spread) the bound only costs (27.8 -> 31.7
+// us at 96^2 x 24 x 150), unless the launch is chained to the kernel before it: then
+// its CTAs start in the filter's tail, and the bound keeps them from piling up on the
+// SMs that are free first (194 against 162 us for a volume of 128^3 x 180 without it).
+// Measured, FBP: 23.4 -> 21.4 us at 64^2 x 64 x 101, 43.8 -> 40.6 at 128^2 x 32 x 201,
+// 41.8 -> 39.6 at 200^2 x 8 x 314. Only for a job by itself (b.alone): beside another
+// stage's kernels the CTAs that wait take their room (256^3 x 360 in slabs 2437 ->
+// 2447 us), and batches gain nothing.
 constexpr int kSmemPerSm = 228 * 1024, kSmemPerCta = 1024;  // of an SM; what each CTA takes besides
-constexpr int smem_for(int own, int per_sm) {
-    const int floor = kSmemPerSm / (per_sm + 1) - kSmemPerCta + 128;  // per_sm + 1 CTAs do not fit
+constexpr size_t smem_for(size_t own, int per_sm) {
+    const size_t floor = kSmemPerSm / (per_sm + 1) - kSmemPerCta + 128;  // per_sm + 1 CTAs do not fit
     return own > floor ? own : floor;
-}
-template <class C>
-size_t item_smem(const BpBatch& b) {
-    const int own = static_cast<int>(sizeof(BpSmem<C>));
-    return static_cast<size_t>(b.per_sm >= 1 && b.per_sm < C::MINB ? smem_for(own, b.per_sm) : own);
 }
 
 template <class C>
 cudaError_t set_smem() {
-    const int bytes = smem_for(static_cast<int>(sizeof(BpSmem<C>)), 1);
+    const int bytes = static_cast<int>(smem_for(sizeof(BpSmem<C>), 1));
     cudaError_t e = cudaFuncSetAttribute(k_backproject<C, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_backproject<C, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -698,27 +699,29 @@ cudaError_t set_smem() {
     return e;
 }
 
-// These launches wait for the kernel before them to end (they are not chained):
-// blocks that start while the filter's last ones still hold their SMs pile up on
-// the SMs that are free first, and stay there for the whole angle loop (194
-// against 162 us for a volume of 128^3 x 180, 225 against 197 us for a slice of
-// 256^2 x 360).
+template <class C, int MODE>
+cudaError_t launch_items(const BpBatch& b, unsigned* d_err, cudaStream_t st) {
+    const dim3 grid(static_cast<unsigned>(b.total));
+    const bool few = b.per_sm >= 1 && b.per_sm < C::MINB;
+    const size_t own = sizeof(BpSmem<C>), smem = few && (b.alone || b.spread) ? smem_for(own, b.per_sm) : own;
+    unsigned* const no_counter = nullptr;
+    if (few && b.alone) return launch_chained(k_backproject<C, MODE>, grid, dim3(THREADS), smem, st, b, no_counter, d_err);
+    k_backproject<C, MODE><<<grid, THREADS, smem, st>>>(b, no_counter, d_err);
+    return cudaGetLastError();
+}
+
 template <class C>
 cudaError_t launch_one(const BpBatch& b, unsigned* d_err, cudaStream_t st) {
     cudaError_t e = set_smem<C>();
     if (e != cudaSuccess) return e;
-    k_backproject<C, 0><<<static_cast<unsigned>(b.total), THREADS, item_smem<C>(b), st>>>(b, nullptr, d_err);
-    return cudaGetLastError();
+    return launch_items<C, 0>(b, d_err, st);
 }
 
 template <class C>
 cudaError_t launch_many(const BpBatch& b, bool persistent, unsigned* d_counter, unsigned* d_err, cudaStream_t st) {
     cudaError_t e = set_smem<C>();
     if (e != cudaSuccess) return e;
-    if (!persistent) {
-        k_backproject<C, 1><<<static_cast<unsigned>(b.total), THREADS, item_smem<C>(b), st>>>(b, nullptr, d_err);
-        return cudaGetLastError();
-    }
+    if (!persistent) return launch_items<C, 1>(b, d_err, st);
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -836,7 +839,8 @@ void bp_number_items(BpBatch& b, int variant, int sms) {
         b.total += static_cast<long long>(J.tiles) * (((J.nz + 3) / 4 + J.zgs - 1) / J.zgs);
     }
     const long long active = pair ? two : one, per_sm = (active + sms - 1) / sms;
-    b.per_sm = per_sm < 16 && b.total > per_sm * sms ? static_cast<int>(per_sm) : 0;
+    b.per_sm = static_cast<int>(std::min(per_sm, 1LL << 20));
+    b.spread = b.total > per_sm * sms;
 }
 
 FiltLayout filt_layout(int sq, int n_out) {
@@ -905,7 +909,7 @@ cudaError_t launch_backproject_batch(const BpBatch& b, int variant, unsigned* d_
 
 cudaError_t launch_backproject(const float4* d_filt, int nz, int na, const FiltLayout& fl,
                                int n_out, Trig trig, const float4* d_stats, int denorm,
-                               float* d_out, unsigned* d_err, cudaStream_t st, int variant, int convention) {
+                               float* d_out, unsigned* d_err, cudaStream_t st, int variant, int convention, bool alone) {
     BpBatch b;
     b.njobs = 1;
     b.job[0] = make_bp_job(d_filt, nz, na, fl, n_out, trig, d_stats, denorm, d_out, variant, convention);
@@ -913,6 +917,7 @@ cudaError_t launch_backproject(const float4* d_filt, int nz, int na, const FiltL
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     bp_number_items(b, variant, sms);
+    b.alone = alone;
     if (b.total > 0x7fffffffLL) return cudaErrorInvalidValue;
     switch (variant) {
     case 1: return launch_one<V1>(b, d_err, st);

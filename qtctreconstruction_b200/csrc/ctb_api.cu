@@ -383,7 +383,8 @@ ctb_status fbp_stage(ctb_ctx* ctx, const float* d_sino, int nz, int na, int bins
     if (ctx->autotune && ctx->bp_variant < 0 && !ctx->tuned.count(bp_bucket(n_out, zs, na)))
         CTB_TRY(tune_backprojection(ctx, d_filt, nz, na, fl, n_out, trig, d_stats, denorm, d_out, &variant, zs));
     CTB_LAUNCH(ctx, launch_backproject(d_filt, nz, na, fl, n_out, trig, d_stats, denorm, d_out,
-                                       ctx->d_err, ctx->stream, variant, ctx->convention));
+                                       ctx->d_err, ctx->stream, variant, ctx->convention,
+                                       shape_depth == 0));  // a slab runs beside its neighbours' stages
     return CTB_OK;
 }
 

@@ -266,7 +266,9 @@ struct BpJob {
 };
 struct BpBatch {
     int njobs = 0;
-    int per_sm = 0;  // most CTAs per SM that balance the items with work, 0: any (bp_number_items)
+    int per_sm = 0;      // items with work per SM, rounded up (bp_number_items)
+    bool spread = false; // more items than per_sm per SM, tiles without work included
+    bool alone = false;  // one job's launch with no other stream's kernels beside it
     long long total = 0;
     BpJob job[kMaxJobs];
 };
@@ -309,7 +311,7 @@ cudaError_t launch_filter_batch(const FiltBatch& b, cudaStream_t st);
 cudaError_t launch_backproject(const float4* d_filt, int nz, int na, const FiltLayout& fl,
                                int n_out, Trig trig, const float4* d_stats, int denorm,
                                float* d_out, unsigned* d_err, cudaStream_t st, int variant = 0,
-                               int convention = kConvSerial);
+                               int convention = kConvSerial, bool alone = true);
 // One CTA whose threads wait, at most `limit_us` microseconds each, on an
 // mbarrier that nothing completes; each records a timeout in *d_err (the
 // timeout path's self-test).
