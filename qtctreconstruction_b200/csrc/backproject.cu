@@ -58,6 +58,7 @@
 // so a job's output is bit-identical alone and in any mix of the same shape.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <type_traits>
 
 #include "ctb_internal.h"
@@ -136,6 +137,11 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
 __device__ __forceinline__ float4 lds128(unsigned a) {
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float2 lds64(unsigned a) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
     return v;
 }
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
@@ -220,9 +226,10 @@ struct BpSmem {
 // (1 - |y|) w[m_v + 1] + max(y, 0) w[m_v + 2] (two taps for v = 0): 11 packed
 // FP32x2 operations per pair of slices and column and 3 to 5 shared loads, where
 // a tap pair per voxel takes 8 of each. ZG groups of four slices share the
-// weights; group p's window lies p WIN bins on.
-template <int P, int ZG, int WIN>
-__device__ __forceinline__ void column_taps(unsigned w, float f1, float as,
+// weights; group p's window lies p WIN bins on. With MASK the voxels whose bit of
+// `keep` is clear get zero weights; the others' sums do not depend on MASK.
+template <int P, int ZG, int WIN, bool MASK>
+__device__ __forceinline__ void column_taps(unsigned w, float f1, float as, unsigned keep,
                                             float2 (&acc)[V][2 * ZG]) {
     constexpr int T = P == 0 ? 3 : P == 3 ? 5 : 4;
     constexpr int m0[V] = {0, 0, P >= 2 ? 1 : 0, P == 0 ? 0 : P == 3 ? 2 : 1};
@@ -236,6 +243,12 @@ __device__ __forceinline__ void column_taps(unsigned w, float f1, float as,
         c[v][0] = fmaxf(-y, 0.0f);
         c[v][1] = 1.0f - fabsf(y);
         c[v][2] = fmaxf(y, 0.0f);
+    }
+    if constexpr (MASK) {
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) c[v][i] = keep & (1u << v) ? c[v][i] : 0.0f;
     }
 #pragma unroll
     for (int m = 0; m < T; ++m) {
@@ -494,12 +507,37 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
             // floor(u) + kRound gives the tap's
             unsigned ra = smem_u32(&S.rec[slot][g]);
             unsigned wa = smem_u32(&S.win[slot][g * ZG][0]) - (static_cast<unsigned>(kRoundBits) << 4);
-            auto run = [&](auto pattern) {
+            // Which voxels of column k take part in an angle whose window reaches a
+            // detector edge: SerialBackend.cpp:229-239 evaluates u = (xx cos - yy sin)
+            // + dc in float without fused multiply-add and keeps the tap pair only
+            // when 0 <= floor(u) and floor(u) + 1 < sq. That decision is reproduced
+            // here exactly; the interpolation itself uses the accurate u.
+            auto in_range = [&](int k, float2 rcs) {
+                const float dcf = static_cast<float>(J.dc);
+                unsigned keep = 0;
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    const int sl = V * col[k] + v;
+                    const int sa = flipped ? (along_x ? TX : TY) - 1 - sl : sl;
+                    const float xs = static_cast<float>(x0 + (along_x ? sa : fast)) - radf;
+                    const float ys = static_cast<float>(y0 + (along_x ? fast : sa)) - radf;
+                    const float us = __fadd_rn(__fsub_rn(__fmul_rn(xs, rcs.x), __fmul_rn(ys, rcs.y)), dcf);
+                    const int is = static_cast<int>(floorf(us));
+                    if (is >= 0 && is + 1 < sq) keep |= 1u << v;
+                }
+                return keep;
+            };
+            // EDGES: some angle of the stage has `edge` set. An angle's sums depend on
+            // its own flag only: what else is in its stage must not change a bit.
+            auto run = [&](auto pattern, auto edges) {
                 constexpr int P = decltype(pattern)::value;
+                constexpr bool EDGES = decltype(edges)::value;
                 float4 rec = lds128(ra);
                 const unsigned end = wa + static_cast<unsigned>((cnt - g + C::SPLIT - 1) / C::SPLIT) * (C::SPLIT * ZG * WIN * 16u);
                 while (wa != end) {
                     const float rf0 = rec.x, rcf = rec.y, ras = rec.z;
+                    const bool edge = EDGES && __float_as_int(rec.w);
+                    const unsigned rest = ra + offsetof(AngleRec, rc);
                     ra += C::SPLIT * sizeof(AngleRec);
                     rec = lds128(ra);  // the next angle's
 #pragma unroll
@@ -507,57 +545,22 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
                         if (NC > 1 && !live[k]) continue;
                         const float u = fmaf(fi, rcf, fmaf(fj[k], ras, rf0));
                         const float tr = __fadd_rd(u, kRound);  // floor(u), no conversion-unit instruction
-                        column_taps<P, ZG, WIN>(wa + (__float_as_uint(tr) << 4), u - (tr - (kRound - 1.0f)), ras,
-                                                acc[k]);
+                        const unsigned keep = edge ? in_range(k, lds64(rest)) : ~0u;
+                        column_taps<P, ZG, WIN, EDGES>(wa + (__float_as_uint(tr) << 4), u - (tr - (kRound - 1.0f)),
+                                                       ras, keep, acc[k]);
                     }
                     wa += C::SPLIT * ZG * WIN * sizeof(float4);
                 }
             };
-            if (meta >> 16) {
-                // SerialBackend.cpp:229-239 evaluates u = (xx cos - yy sin) + dc in
-                // float without fused multiply-add and keeps the tap pair only when
-                // 0 <= floor(u) and floor(u) + 1 < sq; that decision is reproduced
-                // here exactly, the interpolation itself uses the accurate u.
-                const float dcf = static_cast<float>(J.dc);
-                for (int j = g; j < cnt; j += C::SPLIT) {
-                    const AngleRec r = S.rec[slot][j];
-                    const float4* w = S.win[slot][j * ZG];
-#pragma unroll
-                    for (int k = 0; k < NC; ++k) {
-#pragma unroll
-                        for (int v = 0; v < V; ++v) {
-                            const float uv = fmaf(static_cast<float>(v), r.as, fmaf(fi, r.cf, fmaf(fj[k], r.as, r.f0)));
-                            const float fl = floorf(uv);
-                            const int iv = static_cast<int>(fl);
-                            const int sl = V * col[k] + v;
-                            const int sa = flipped ? (along_x ? TX : TY) - 1 - sl : sl;
-                            const float xs = static_cast<float>(x0 + (along_x ? sa : fast)) - radf;
-                            const float ys = static_cast<float>(y0 + (along_x ? fast : sa)) - radf;
-                            const float us = __fadd_rn(__fsub_rn(__fmul_rn(xs, r.rc), __fmul_rn(ys, r.rs)), dcf);
-                            const int is = static_cast<int>(floorf(us));
-                            const bool ok = !r.edge || ((is >= 0) && (is + 1 < sq));
-                            const float w1 = ok ? uv - fl : 0.0f;
-                            const float w0 = ok ? 1.0f - (uv - fl) : 0.0f;
-                            const float2 W0 = make_float2(w0, w0), W1 = make_float2(w1, w1);
-#pragma unroll
-                            for (int p = 0; p < ZG; ++p) {
-                                const float4 lo = w[p * WIN + iv], hi = w[p * WIN + iv + 1];
-                                float2(&A)[NH] = acc[k][v];
-                                A[2 * p] = __ffma2_rn(W1, make_float2(hi.x, hi.y),
-                                                      __ffma2_rn(W0, make_float2(lo.x, lo.y), A[2 * p]));
-                                A[2 * p + 1] = __ffma2_rn(W1, make_float2(hi.z, hi.w),
-                                                          __ffma2_rn(W0, make_float2(lo.z, lo.w), A[2 * p + 1]));
-                            }
-                        }
-                    }
-                }
-            } else {
+            auto run_pattern = [&](auto edges) {
                 const int pat = grp % 4;
-                if (pat == 0) run(std::integral_constant<int, 0>());
-                else if (pat == 1) run(std::integral_constant<int, 1>());
-                else if (pat == 2) run(std::integral_constant<int, 2>());
-                else run(std::integral_constant<int, 3>());
-            }
+                if (pat == 0) run(std::integral_constant<int, 0>(), edges);
+                else if (pat == 1) run(std::integral_constant<int, 1>(), edges);
+                else if (pat == 2) run(std::integral_constant<int, 2>(), edges);
+                else run(std::integral_constant<int, 3>(), edges);
+            };
+            if (meta >> 16) run_pattern(std::true_type());
+            else run_pattern(std::false_type());
         }
         __syncwarp();
         if ((t & 31) == 0) mbar_arrive(&S.empty[slot]);
