@@ -175,11 +175,12 @@ ctb_status ctb_probe_smem_bandwidth(ctb_ctx* ctx, double* gbs);
  * (CUDABackend.cu:37-43, HybridBackend.cu:44-65); here every device-side wait
  * is bounded (2 s of the GPU's global timer) and a wait that gives up makes
  * the call return CTB_ERR_TIMEOUT with the context still usable.
- * ctb_selftest_bounded_wait runs that path on purpose: one CTA waits, at most
- * `limit_us` microseconds (1 .. 2e6), on a barrier that nothing completes (no
- * copy is in flight), records the timeout and returns. It returns
- * CTB_ERR_TIMEOUT when the path works (CTB_OK would mean the wait was not
- * bounded).
+ * ctb_selftest_bounded_wait runs that path on purpose, with waits of at most
+ * limit_us microseconds (1 .. 2000000): a backprojection tile one of whose stages
+ * is never copied (code 1), then one CTA that waits on a barrier nothing
+ * completes (code 16). Both record the timeout and return; it returns
+ * CTB_ERR_TIMEOUT when the path works (CTB_OK would mean the waits were not
+ * bounded), with the codes of both, 17, in ctb_last_error.
  * ctb_set_fault_injection (host side, for tests): with slab >= 0 the next
  * ctb_reconstruct_volume calls fail with CTB_ERR_CUDA after queuing that
  * slab's copy and forward stage, with earlier slabs still in flight; such a

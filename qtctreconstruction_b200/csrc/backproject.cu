@@ -57,6 +57,7 @@
 // atomic counter. An item's arithmetic depends only on its job and tile shape,
 // so a job's output is bit-identical alone and in any mix of the same shape.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstddef>
 #include <type_traits>
@@ -156,19 +157,22 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+constexpr unsigned long long kWaitLimitNs = 2000000000ull;
 // Bounded wait: gives up once `limit_ns` nanoseconds of the GPU's global timer
 // have passed since the first unsuccessful poll (2 s in the kernels; a poll may
 // itself suspend for a hardware-defined interval, so the bound is on time, with
-// 2^22 polls as a second cap), and reports `code` through the device error word.
+// 2^22 polls as a second cap), and reports `code` through the device error word. With
+// `stop` it also gives up, reporting nothing, once another wait of the block did.
 __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsigned parity,
                                                   unsigned* err,
-                                                  unsigned long long limit_ns = 2000000000ull,
-                                                  unsigned code = 1u) {
+                                                  unsigned long long limit_ns = kWaitLimitNs,
+                                                  unsigned code = 1u, const volatile int* stop = nullptr) {
     if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
     for (unsigned it = 0; it < (1u << 22); ++it) {
         __nanosleep(32);  // leave the issue slots to the warps that work
         if (mbar_try_wait(bar, parity)) return true;
+        if (stop && *stop) return false;
         if (global_ns() - t0 > limit_ns) break;
     }
     if (err) atomicOr(err, code);
@@ -209,11 +213,18 @@ struct BpSmem {
     float2 ex[C::SPLIT * C::TX * C::TY];     // exchange of accumulators between threads
     AngleRec rec[NST][C::SW + C::SPLIT];     // a record is read ahead of its use
     unsigned long long full[NST], empty[NST];
-    int meta[NST];                           // stage: angles | group << 8 | some angle has `edge` set << 16
+    int meta[NST];                           // stage: angles | some angle has `edge` set << 8
+    unsigned sent[NST];                      // stages whose copies were issued into the slot
     int first[kBpGroups];                    // first stage of each group of the angle order
     int start[kBpGroups + 1];                // first angle of each group; na
     int total;                               // stages of the item
     int dead;                                // a wait gave up
+};
+
+// A stage whose copies the self-test leaves out, and its waits' limit.
+struct BpLost {
+    int stage;
+    unsigned long long limit_ns;
 };
 
 // One column of V = 4 voxels at one angle. w: shared address of the window bin of the column's
@@ -271,10 +282,13 @@ __device__ __forceinline__ void column_taps(unsigned w, float f1, float as, unsi
 
 // Backproject one tile (x0, y0) of ZG slice groups from zg on of job J. `stages`
 // counts the stages this CTA has consumed so far (mbarrier phases continue
-// across items). Returns false when a bounded wait gave up (block-uniform).
-template <class C, int ZG>
+// across items). Returns false when a bounded wait gave up (block-uniform): from
+// then on no warp issues a copy, waits or reads a window, but all go through the
+// stages' barriers of the block, whose place follows from the angle order alone, and
+// the copies under way are waited for before the return.
+template <class C, int ZG, bool LOST = false>
 __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, int x0, int y0, unsigned& stages,
-                                        unsigned* err) {
+                                        unsigned* err, BpLost lost = {}) {
     constexpr int TX = C::TX, TY = C::TY, WIN = C::WIN, NC = C::NC;
     constexpr int SA = C::SW / ZG;           // angles per stage
     constexpr int NST = C::NST, AHEAD = C::AHEAD;
@@ -332,6 +346,14 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
     }
     __syncthreads();
     const int total = S.total;
+    // the group of a stage: the last one that starts at or before it
+    const int my_first = lane < kBpGroups ? S.first[lane] : INT_MAX;
+    auto group_of = [&](int i) { return __popc(__ballot_sync(0xffffffffu, my_first <= i)) - 1; };
+    auto wait = [&](unsigned long long* bar, unsigned parity) {
+        const bool ok = mbar_wait_bounded(bar, parity, err, LOST ? lost.limit_ns : kWaitLimitNs, 1u, &S.dead);
+        if (!ok) *static_cast<volatile int*>(&S.dead) = 1;
+        return ok;
+    };
 
     // One warp fills the item's stage i (the CTA's stage s).
     // Its slot was last used NST stages ago: every warp arrived on `empty` after
@@ -340,21 +362,12 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
         const int slot = s % NST;
         const unsigned use = s / NST;
         bool ok = *static_cast<volatile int*>(&S.dead) == 0;
-        if (ok && use > 0 && !mbar_wait_bounded(&S.empty[slot], (use - 1) & 1, err)) ok = false;
-        ok = __all_sync(0xffffffffu, ok);
-        // the last group that starts at or before stage i
-        const int grp = __popc(__ballot_sync(0xffffffffu, lane < kBpGroups && S.first[lane & (kBpGroups - 1)] <= i)) - 1;
+        if (ok && use > 0) ok = wait(&S.empty[slot], (use - 1) & 1);
+        if (!__all_sync(0xffffffffu, ok)) return;  // nothing is copied any more
+        const int grp = group_of(i);
         const int pos = S.start[grp] + (i - S.first[grp]) * SA;
         const int cnt = min(SA, S.start[grp + 1] - pos);
         const bool along = grp < kBpGroups / 2, flip = (grp / 4) & 1;
-        if (!ok) {  // nothing is copied any more; the consumers' waits still end
-            if (lane == 0) {
-                *static_cast<volatile int*>(&S.dead) = 1;
-                S.meta[slot] = SA;
-                mbar_expect_tx(&S.full[slot], 0);
-            }
-            return;
-        }
         int a = 0, ws = 0, edge = 0;
         if (lane < cnt) {
             a = J.trig.order[pos + lane];
@@ -383,12 +396,16 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
             S.rec[slot][lane] = r;
         }
         edge = __any_sync(0xffffffffu, edge);
-        if (lane == 0) S.meta[slot] = cnt | grp << 8 | (edge ? 1 << 16 : 0);
+        const bool send = !LOST || i != lost.stage;
+        if (lane == 0) {
+            S.meta[slot] = cnt | (edge ? 1 << 8 : 0);
+            if (send) S.sent[slot] = use + 1;
+        }
         __syncwarp();
         // the arrival publishes the records; the copies complete the stage
         if (lane == 0) mbar_expect_tx(&S.full[slot], static_cast<unsigned>(cnt * ZG * WIN * sizeof(float4)));
         __syncwarp();
-        if (lane < cnt) {
+        if (lane < cnt && send) {
             const float4* row = J.filt + (static_cast<long long>(zg) * na + a) * J.pitch + J.guard + ws;
 #pragma unroll
             for (int p = 0; p < ZG; ++p)
@@ -484,13 +501,10 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
     for (int i = 0; i < total; ++i, ++stages) {
         const int slot = stages % NST;
         if (warp == i % (THREADS / 32) && i + AHEAD < total) produce(stages + AHEAD, i + AHEAD);
-        // A failed wait leaves stale window data; the block then stops as a
-        // whole at the end of the item (the decision is block-uniform).
-        if (!mbar_wait_bounded(&S.full[slot], (stages / NST) & 1, err)) {
-            landed = false;
-            *static_cast<volatile int*>(&S.dead) = 1;
-        }
-        const int meta = S.meta[slot], cnt = meta & 0xff, grp = (meta >> 8) & 0xff;
+        // A failed wait leaves stale records and windows: the warp takes nothing of
+        // them, and the block stops as a whole at the end of the item.
+        landed = landed && wait(&S.full[slot], (stages / NST) & 1);
+        const int grp = group_of(i);
         if (along_x && grp >= kBpGroups / 2) exchange();
         if (flipped != (((grp / 4) & 1) != 0)) flip_columns();
         const float fi = static_cast<float>(fast);
@@ -501,7 +515,8 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
             fj[k] = static_cast<float>(V * col[k]);
             some |= live[k];
         }
-        if (some && landed && g < cnt) {
+        const int meta = landed ? S.meta[slot] : 0, cnt = meta & 0xff;
+        if (some && g < cnt) {
             // 32-bit shared addresses of this group's first record and window;
             // the window's is offset so that adding 16 times the bits of
             // floor(u) + kRound gives the tap's
@@ -559,13 +574,17 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
                 else if (pat == 2) run(std::integral_constant<int, 2>(), edges);
                 else run(std::integral_constant<int, 3>(), edges);
             };
-            if (meta >> 16) run_pattern(std::true_type());
+            if (meta >> 8) run_pattern(std::true_type());
             else run_pattern(std::false_type());
         }
         __syncwarp();
-        if ((t & 31) == 0) mbar_arrive(&S.empty[slot]);
+        if ((t & 31) == 0 && landed) mbar_arrive(&S.empty[slot]);
     }
-    if (!__syncthreads_and(landed)) return false;
+    if (!__syncthreads_and(landed)) {
+        if (t < NST && S.sent[t] > 0) mbar_wait_bounded(&S.full[t], (S.sent[t] - 1) & 1, err);
+        __syncthreads();
+        return false;
+    }
     if (along_x) exchange();
     if (flipped) flip_columns();
     if constexpr (C::SPLIT > 1) {
@@ -616,6 +635,19 @@ __device__ __forceinline__ bool bp_item(BpSmem<C>& S, const BpJob& J, int zi, in
     return bp_tile<C, 1>(S, J, zg, x0, y0, stages, err);
 }
 
+template <class C>
+__device__ __forceinline__ void bp_init(BpSmem<C>& S) {
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < C::NST; ++b) {
+            mbar_init(&S.full[b], 1);
+            mbar_init(&S.empty[b], THREADS / 32);
+            S.sent[b] = 0;
+        }
+        S.dead = 0;
+        mbar_fence_init();
+    }
+}
+
 // MODE 0: one job, one CTA per item (job 0 indexed statically keeps its fields
 // constant-bank operands). MODE 1: many jobs, one CTA per item, the job found
 // from blockIdx.x. MODE 2: a persistent grid whose thread 0 draws items from
@@ -627,14 +659,7 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
     extern __shared__ __align__(128) unsigned char smem_raw[];
     BpSmem<C>& S = *reinterpret_cast<BpSmem<C>*>(smem_raw);
     __shared__ int s_item;
-    if (threadIdx.x == 0) {
-        for (int b = 0; b < C::NST; ++b) {
-            mbar_init(&S.full[b], 1);
-            mbar_init(&S.empty[b], THREADS / 32);
-        }
-        S.dead = 0;
-        mbar_fence_init();
-    }
+    bp_init(S);
     chain_wait();  // lets the next call's first kernel start in this one's tail
     unsigned stages = 0;
     if constexpr (MODE == 0) {
@@ -669,6 +694,20 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
             __syncthreads();  // shared state of this item is dead before the next item's staging
         }
     }
+}
+
+// Self-test of a lost copy: one item of two slice groups, one of whose stages is
+// never copied. Every warp's wait for it gives up after `limit_us` microseconds or
+// as soon as another's did, and the block ends as it does after such a fault.
+template <class C>
+__global__ void __launch_bounds__(THREADS, C::MINB) k_bp_selftest(const __grid_constant__ BpBatch batch, int stage,
+                                                                  unsigned limit_us, unsigned* err) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    BpSmem<C>& S = *reinterpret_cast<BpSmem<C>*>(smem_raw);
+    bp_init(S);
+    __syncthreads();
+    unsigned stages = 0;
+    bp_tile<C, 2, true>(S, batch.job[0], 0, 0, 0, stages, err, BpLost{stage, 1000ull * limit_us});
 }
 
 // Launches with one CTA per item whose items with work need fewer CTAs per SM
@@ -745,6 +784,17 @@ BpShape shape_of() {
 
 cudaError_t launch_wait_selftest(unsigned limit_us, unsigned* d_err, cudaStream_t st) {
     k_wait_selftest<<<1, 64, 0, st>>>(limit_us, d_err);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bp_selftest(const float4* d_filt, int na, const FiltLayout& fl, int n_out, Trig trig, float* d_out,
+                               unsigned limit_us, unsigned* d_err, cudaStream_t st) {
+    BpBatch b;
+    b.job[0] = make_bp_job(d_filt, 8, na, fl, n_out, trig, nullptr, CTB_DENORM_NONE, d_out, 0, kConvSerial);
+    const int smem = static_cast<int>(sizeof(BpSmem<V0>));
+    const cudaError_t e = cudaFuncSetAttribute(k_bp_selftest<V0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    k_bp_selftest<V0><<<1, THREADS, smem, st>>>(b, 3, limit_us, d_err);
     return cudaGetLastError();
 }
 

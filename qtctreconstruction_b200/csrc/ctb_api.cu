@@ -793,6 +793,17 @@ ctb_status ctb_selftest_bounded_wait(ctb_ctx* ctx, unsigned limit_us) {
     if (!ctx || limit_us == 0 || limit_us > 2000000u) return CTB_ERR_INVALID;
     Guard g(ctx);
     CTB_TRY(check_error_word(ctx));  // a stale error word is not this test's
+    // a backprojection tile of 32^2 with angles along both axes, so that the block's
+    // exchange of sums lies behind the lost stage
+    const int n = 32, na = 180;
+    const FiltLayout fl = filt_layout(pad_geometry(n).sq, n);
+    const size_t filt = static_cast<size_t>(2) * na * fl.pitch;
+    CTB_WS(ctx, d_filt, float4, "selftest", filt + static_cast<size_t>(8) * n * n / 4);
+    Trig trig;
+    CTB_TRY(trig_table(ctx, nullptr, na, &trig));
+    CTB_CUDA(ctx, cudaMemsetAsync(d_filt, 0, sizeof(float4) * filt, ctx->stream));
+    CTB_LAUNCH(ctx, launch_bp_selftest(d_filt, na, fl, n, trig, reinterpret_cast<float*>(d_filt + filt), limit_us,
+                                       ctx->d_err, ctx->stream));
     CTB_LAUNCH(ctx, launch_wait_selftest(limit_us, ctx->d_err, ctx->stream));
     return check_error_word(ctx);
 }

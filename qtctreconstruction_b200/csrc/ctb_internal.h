@@ -316,6 +316,11 @@ cudaError_t launch_backproject(const float4* d_filt, int nz, int na, const FiltL
 // mbarrier that nothing completes; each records a timeout in *d_err (the
 // timeout path's self-test).
 cudaError_t launch_wait_selftest(unsigned limit_us, unsigned* d_err, cudaStream_t st);
+// One item of the backprojector (eight slices of a tile, 32x32 shape) whose fourth
+// stage of angles is never copied; its waits give up after `limit_us` microseconds
+// and record code 1 in *d_err.
+cudaError_t launch_bp_selftest(const float4* d_filt, int na, const FiltLayout& fl, int n_out, Trig trig, float* d_out,
+                               unsigned limit_us, unsigned* d_err, cudaStream_t st);
 cudaError_t launch_point_count(const float* d_vol, long long total, float thr,
                                unsigned* d_block_counts, int blocks, cudaStream_t st);
 cudaError_t launch_point_write(const float* d_vol, int nx, int ny, long long total, float thr,
