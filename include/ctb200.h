@@ -125,7 +125,9 @@ ctb_status ctb_set_filter_mode(ctb_ctx* ctx, int mode);
  * voxel's angles in the same order as shape 0 and so give its result bit for
  * bit. (A chunk is half the ring of staged windows, one window per angle and
  * group of four slices.) Without tuning a job gets a shape from its size alone:
- * 32x32, or 32x16 or 16x16 where its tiles would leave SMs idle. With the autotuner
+ * 32x32, or 32x16 or 16x16 where its tiles would leave SMs idle; jobs of few angles
+ * (24, or up to 64 where their tiles leave SMs idle) take such a tile in a kernel of
+ * their own, which is neither tuned nor forced. With the autotuner
  * on, the first job of each size bucket {ceil(n / 64), ceil(angles / 180),
  * floor(log2(ceil(depth / 4)))} times every shape on its own data (that call
  * synchronises) and the fastest is kept for the bucket; batches use a tuned

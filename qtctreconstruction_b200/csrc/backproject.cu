@@ -52,6 +52,8 @@
 // at the end, so that a thread always has columns to share taps in and its
 // serial chain of angles is short.
 //
+// Jobs of few angles (bp_default_variant) have a tile function without columns.
+//
 // One kernel serves both shapes of work: a single job with one CTA per item,
 // or a batch of jobs (BpBatch) on a persistent grid that takes items from an
 // atomic counter. An item's arithmetic depends only on its job and tile shape,
@@ -83,7 +85,7 @@ constexpr int V = 4;
 template <int TX_, int TY_, int CA_, int WIN_, int SW_, int NST_, int MINB_, bool PAIR_>
 struct Shape {
     static constexpr int TX = TX_, TY = TY_, CA = CA_, WIN = WIN_, MINB = MINB_;
-    static constexpr bool PAIR = PAIR_;
+    static constexpr bool PAIR = PAIR_, FEW = false;
     // Stages, and how many the producer works ahead: it refills the slot of two
     // stages back, so a warp may lag one stage without holding it up (refilling
     // the last stage's slot made every producer wait for the slowest warp: 13.3
@@ -107,6 +109,20 @@ using V2 = Shape<32, 16, 32, 40, 24, 4, 3, true>;  // half-height tiles: twice t
 using V3 = Shape<16, 16, 32, 28, 24, 4, 3, true>;  // small tiles for small slices
 using V4 = Shape<32, 32, 16, 48, 12, 3, 3, true>;  // the general shape with half the ring
 using V5 = Shape<32, 32, 64, 48, 32, 4, 2, true>;  // the general shape with twice the ring (half the stages)
+
+// A tile shape of jobs with few angles (few_tile): TX x TY voxels of four slices, VPT voxels per thread along x (TX / VPT apart), 32 angles per staged
+// chunk.
+template <int TX_, int TY_, int VPT_, int WIN_>
+struct Few {
+    static constexpr int TX = TX_, TY = TY_, VPT = VPT_, CA = 32, WIN = WIN_, MINB = 4;
+    static constexpr bool PAIR = false, FEW = true;
+    static constexpr int XS = TX / VPT;
+    static_assert(XS * TY == THREADS, "256 threads per CTA");
+    static_assert(WIN <= kBpWindowMax, "window within the filtered-row guard");
+};
+using F0 = Few<32, 32, 4, 52>;
+using F2 = Few<32, 16, 2, 40>;
+using F3 = Few<16, 16, 1, 28>;
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
     return static_cast<unsigned>(__cvta_generic_to_shared(p));
@@ -624,8 +640,231 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
     return true;
 }
 
+// ------------------------------------------------------------ few angles
+// A job of few angles gains nothing from the columns: its 16 groups make as many
+// nearly empty stages, each with another of the unrolled tap patterns, and the
+// exchange of sums and 3 CTAs per SM stand against writing the output. So each
+// voxel interpolates on its own between two taps, in the angles' given order, with
+// four CTAs per SM (FBP of 512^2 x 64: 73.7 -> 60.6 us at 8 angles, 103.3 -> 89.3 at 16).
+struct FewRec {
+    float f0;      // tile-origin u minus window start
+    float c, s;
+    int edge;      // the window reaches a detector edge: decide taps like the reference
+    float rc, rs;  // the reference's float cos/sin (edge decisions only)
+    int pad[2];
+};
+template <class C>
+struct FewSmem {
+    float4 win[2][C::CA][C::WIN];
+    FewRec rec[2][C::CA];
+    unsigned long long bar[2];
+};
+template <class C>
+using SmemOf = std::conditional_t<C::FEW, FewSmem<C>, BpSmem<C>>;
+
+template <class C>
+__device__ __forceinline__ void bp_init(FewSmem<C>& S) {
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < 2; ++b) mbar_init(&S.bar[b], 1);
+        mbar_fence_init();
+    }
+}
+
+// Backproject one tile (x0, y0) of slice group zg of job J. `chunks` counts the
+// chunks this CTA has consumed so far (mbarrier phases continue across items).
+// Returns false when a bounded wait gave up (block-uniform), the copies under way
+// waited for.
+template <class C>
+__device__ __forceinline__ bool few_tile(FewSmem<C>& S, const BpJob& J, int zg, int x0, int y0, unsigned& chunks,
+                                         unsigned* err) {
+    constexpr int TX = C::TX, TY = C::TY, VPT = C::VPT, XS = C::XS, CA = C::CA, WIN = C::WIN;
+    const int t = threadIdx.x;
+    const int lx = t % XS, ly = t / XS;
+    const int n = J.n, nz = J.nz, na = J.na, sq = J.sq;
+    const double ctr = J.ctr;  // voxel-grid centre (the mask radius too)
+    const float radf = static_cast<float>(ctr);
+
+    float add[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int z = 4 * zg + j;
+        float a = 0.0f;
+        if (J.stats && J.denorm != CTB_DENORM_NONE && z < nz) {
+            const float4 st = J.stats[z];
+            // CUDABackend.cu:676-681 adds the minimum only when max > min
+            a = (J.denorm == CTB_DENORM_CUDA && !(st.y - st.x > 0.0f)) ? 0.0f : st.x;
+        }
+        add[j] = a;
+    }
+
+    // Tiles entirely outside the reconstruction circle hold only the offset.
+    {
+        const int xe = min(x0 + TX - 1, n - 1), ye = min(y0 + TY - 1, n - 1);
+        const double dx = fmax(0.0, fmax(x0 - ctr, ctr - xe));
+        const double dy = fmax(0.0, fmax(y0 - ctr, ctr - ye));
+        if (dx * dx + dy * dy > ctr * ctr) {
+            const int y = y0 + ly;
+#pragma unroll
+            for (int k = 0; k < VPT; ++k) {
+                const int x = x0 + lx + XS * k;
+                if (x >= n || y >= n) continue;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int z = 4 * zg + j;
+                    if (z < nz) J.out[(static_cast<long long>(z) * n + y) * n + x] = add[j];
+                }
+            }
+            return true;
+        }
+    }
+
+    const double dcd = J.dc;
+    const float dcf = static_cast<float>(J.dc);
+    const double ox = static_cast<double>(x0) - ctr, oy = static_cast<double>(y0) - ctr;
+    const float4* plane = J.filt + static_cast<long long>(zg) * na * J.pitch;
+    const int nch = (na + CA - 1) / CA;
+
+    auto issue = [&](int c, int b) {
+        const int a0 = c * CA;
+        const int cnt = min(CA, na - a0);
+        if (t < cnt) {
+            const int a = a0 + t;
+            const double2 tc = J.trig.cs[a];
+            const float2 tf = J.trig.csf[a];
+            const double uo = ox * tc.x - oy * tc.y + dcd;
+            const double umin = uo + fmin(0.0, (TX - 1) * tc.x) + fmin(0.0, -(TY - 1) * tc.y);
+            const double umax = uo + fmax(0.0, (TX - 1) * tc.x) + fmax(0.0, -(TY - 1) * tc.y);
+            const int ws = static_cast<int>(floor(umin)) - 1;
+            FewRec r;
+            r.f0 = static_cast<float>(uo - ws);
+            r.c = static_cast<float>(tc.x);
+            r.s = static_cast<float>(tc.y);
+            r.rc = tf.x;
+            r.rs = tf.y;
+            // taps near bin 0 or bin sq-1: the reference's float u decides them
+            // (the CUDA backend's per-tap bounds need no rule: bins outside
+            // [0, sq) are zeros of the guard)
+            r.edge = (J.edge_rule && (umin < 2.0 || umax > sq - 3.0)) ? 1 : 0;
+            r.pad[0] = r.pad[1] = 0;
+            S.rec[b][t] = r;
+            bulk_load(&S.win[b][t][0], plane + static_cast<long long>(a) * J.pitch + J.guard + ws,
+                      WIN * sizeof(float4), &S.bar[b]);
+        }
+        if (t == 0) mbar_expect_tx(&S.bar[b], static_cast<unsigned>(cnt * WIN * sizeof(float4)));
+    };
+
+    float4 acc[VPT];
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float fx = static_cast<float>(lx), fy = static_cast<float>(ly);
+    // positions inside the reconstruction circle (SerialBackend.cpp:220-224);
+    // the others are written as the offset only, so their taps are never loaded
+    unsigned inside_mask = 0;
+    {
+        const float yy = static_cast<float>(y0 + ly) - radf;
+#pragma unroll
+        for (int k = 0; k < VPT; ++k) {
+            const float xx = static_cast<float>(x0 + lx + XS * k) - radf;
+            if (!(xx * xx + yy * yy > radf * radf)) inside_mask |= 1u << k;
+        }
+    }
+
+    // all buffers are idle between items: chunk g of this CTA uses buffer g & 1
+    issue(0, chunks & 1);
+    __syncthreads();
+    for (int c = 0; c < nch; ++c) {
+        const unsigned g = chunks + c;
+        const int b = g & 1;
+        if (c + 1 < nch) issue(c + 1, (g + 1) & 1);
+        // A failed wait leaves stale window data; the block then stops as a
+        // whole at the barrier below (the decision is block-uniform).
+        const bool landed = mbar_wait_bounded(&S.bar[b], (g >> 1) & 1, err);
+        const int cnt = min(CA, na - c * CA);
+        for (int j = 0; j < cnt; ++j) {
+            const FewRec r = S.rec[b][j];
+            const float4* w = S.win[b][j];
+            const float ub = fmaf(fx, r.c, fmaf(-fy, r.s, r.f0));
+            const float c8 = static_cast<float>(XS) * r.c;
+            if (!r.edge) {
+                // i = floor(u) by rounding u - 1/2 with the kRound addition (no
+                // conversion-unit instructions); at an exact tie u = i + 1 the taps
+                // shift to (i, i+1) with weights (0, 1), the same value
+                const float ubh = ub - 0.5f;
+#pragma unroll
+                for (int k = 0; k < VPT; ++k) {
+                    if (!(inside_mask & (1u << k))) continue;
+                    const float uh = fmaf(static_cast<float>(k), c8, ubh);
+                    const float tr = uh + kRound;
+                    const int i = __float_as_int(tr) - kRoundBits;
+                    const float d = uh - (tr - kRound);  // frac(u) - 1/2
+                    const float w1 = d + 0.5f;
+                    const float w0 = 0.5f - d;
+                    const float4 lo = w[i], hi = w[i + 1];
+                    acc[k].x = fmaf(w1, hi.x, fmaf(w0, lo.x, acc[k].x));
+                    acc[k].y = fmaf(w1, hi.y, fmaf(w0, lo.y, acc[k].y));
+                    acc[k].z = fmaf(w1, hi.z, fmaf(w0, lo.z, acc[k].z));
+                    acc[k].w = fmaf(w1, hi.w, fmaf(w0, lo.w, acc[k].w));
+                }
+            } else {
+                // SerialBackend.cpp:229-239 evaluates u = (xx cos - yy sin) + dc in
+                // float without fused multiply-add and keeps the tap pair only when
+                // 0 <= floor(u) and floor(u) + 1 < sq; that decision is reproduced
+                // here exactly, the interpolation itself uses the accurate u.
+#pragma unroll
+                for (int k = 0; k < VPT; ++k) {
+                    if (!(inside_mask & (1u << k))) continue;
+                    const float u = fmaf(static_cast<float>(k), c8, ub);
+                    const float fl = floorf(u);
+                    const int i = static_cast<int>(fl);
+                    const float xs = static_cast<float>(x0 + lx + XS * k) - radf;
+                    const float ys = static_cast<float>(y0 + ly) - radf;
+                    const float us = __fadd_rn(__fsub_rn(__fmul_rn(xs, r.rc), __fmul_rn(ys, r.rs)), dcf);
+                    const int is = static_cast<int>(floorf(us));
+                    const bool ok = (is >= 0) && (is + 1 < sq);
+                    const float w1 = ok ? u - fl : 0.0f;
+                    const float w0 = ok ? 1.0f - (u - fl) : 0.0f;
+                    const float4 lo = w[i], hi = w[i + 1];
+                    acc[k].x = fmaf(w1, hi.x, fmaf(w0, lo.x, acc[k].x));
+                    acc[k].y = fmaf(w1, hi.y, fmaf(w0, lo.y, acc[k].y));
+                    acc[k].z = fmaf(w1, hi.z, fmaf(w0, lo.z, acc[k].z));
+                    acc[k].w = fmaf(w1, hi.w, fmaf(w0, lo.w, acc[k].w));
+                }
+            }
+        }
+        if (!__syncthreads_and(landed)) {
+            if (t == 0) {
+                mbar_wait_bounded(&S.bar[b], (g >> 1) & 1, err);
+                if (c + 1 < nch) mbar_wait_bounded(&S.bar[b ^ 1], ((g + 1) >> 1) & 1, err);
+            }
+            __syncthreads();
+            return false;
+        }
+    }
+    chunks += nch;
+
+    const int y = y0 + ly;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+        const int x = x0 + lx + XS * k;
+        if (x >= n || y >= n) continue;
+        const bool inside = inside_mask & (1u << k);
+        const float v[4] = {acc[k].x, acc[k].y, acc[k].z, acc[k].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int z = 4 * zg + j;
+            if (z < nz) J.out[(static_cast<long long>(z) * n + y) * n + x] = (inside ? v[j] : 0.0f) + add[j];
+        }
+    }
+    return true;
+}
+
 // One item: the tile (x0, y0) of slice groups zg J.zgs ... of job J (a pair, or
 // one group where a pair would pass the last slice).
+template <class C>
+__device__ __forceinline__ bool bp_item(FewSmem<C>& S, const BpJob& J, int zg, int x0, int y0, unsigned& chunks,
+                                        unsigned* err) {
+    return few_tile<C>(S, J, zg, x0, y0, chunks, err);
+}
 template <class C>
 __device__ __forceinline__ bool bp_item(BpSmem<C>& S, const BpJob& J, int zi, int x0, int y0, unsigned& stages,
                                         unsigned* err) {
@@ -657,7 +896,7 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
                                                                   unsigned* __restrict__ counter,
                                                                   unsigned* __restrict__ err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    BpSmem<C>& S = *reinterpret_cast<BpSmem<C>*>(smem_raw);
+    SmemOf<C>& S = *reinterpret_cast<SmemOf<C>*>(smem_raw);
     __shared__ int s_item;
     bp_init(S);
     chain_wait();  // lets the next call's first kernel start in this one's tail
@@ -667,7 +906,7 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
         const BpJob& J = batch.job[0];
         const int zg = blockIdx.x / J.tiles;
         const int tl = blockIdx.x - zg * J.tiles;
-        bp_item<C>(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, stages, err);
+        bp_item(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, stages, err);
     } else if constexpr (MODE == 1) {
         __syncthreads();
         const int item = blockIdx.x;
@@ -677,7 +916,7 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
         const int local = item - static_cast<int>(J.first);
         const int zg = local / J.tiles;
         const int tl = local - zg * J.tiles;
-        bp_item<C>(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, stages, err);
+        bp_item(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, stages, err);
     } else {
         for (;;) {
             if (threadIdx.x == 0) s_item = static_cast<int>(atomicAdd(counter, 1u));
@@ -690,7 +929,7 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
             const int local = item - static_cast<int>(J.first);
             const int zg = local / J.tiles;
             const int tl = local - zg * J.tiles;
-            if (!bp_item<C>(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, stages, err)) break;
+            if (!bp_item(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, stages, err)) break;
             __syncthreads();  // shared state of this item is dead before the next item's staging
         }
     }
@@ -732,7 +971,7 @@ constexpr size_t smem_for(size_t own, int per_sm) {
 
 template <class C>
 cudaError_t set_smem() {
-    const int bytes = static_cast<int>(smem_for(sizeof(BpSmem<C>), 1));
+    const int bytes = static_cast<int>(smem_for(sizeof(SmemOf<C>), 1));
     cudaError_t e = cudaFuncSetAttribute(k_backproject<C, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_backproject<C, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -745,7 +984,7 @@ template <class C, int MODE>
 cudaError_t launch_items(const BpBatch& b, unsigned* d_err, cudaStream_t st) {
     const dim3 grid(static_cast<unsigned>(b.total));
     const bool few = b.per_sm >= 1 && b.per_sm < C::MINB;
-    const size_t own = sizeof(BpSmem<C>), smem = few && (b.alone || b.spread) ? smem_for(own, b.per_sm) : own;
+    const size_t own = sizeof(SmemOf<C>), smem = few && (b.alone || b.spread) ? smem_for(own, b.per_sm) : own;
     unsigned* const no_counter = nullptr;
     if (few && b.alone) return launch_chained(k_backproject<C, MODE>, grid, dim3(THREADS), smem, st, b, no_counter, d_err);
     k_backproject<C, MODE><<<grid, THREADS, smem, st>>>(b, no_counter, d_err);
@@ -767,11 +1006,11 @@ cudaError_t launch_many(const BpBatch& b, bool persistent, unsigned* d_counter, 
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backproject<C, 2>, THREADS, sizeof(BpSmem<C>));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backproject<C, 2>, THREADS, sizeof(SmemOf<C>));
     const long long grid = std::min<long long>(b.total, static_cast<long long>(sms) * (per_sm > 0 ? per_sm : 1));
     e = cudaMemsetAsync(d_counter, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
-    k_backproject<C, 2><<<static_cast<unsigned>(grid), THREADS, sizeof(BpSmem<C>), st>>>(b, d_counter, d_err);
+    k_backproject<C, 2><<<static_cast<unsigned>(grid), THREADS, sizeof(SmemOf<C>), st>>>(b, d_counter, d_err);
     return cudaGetLastError();
 }
 
@@ -805,6 +1044,9 @@ BpShape bp_shape(int variant) {
     case 3: return shape_of<V3>();
     case 4: return shape_of<V4>();
     case 5: return shape_of<V5>();
+    case 6: return shape_of<F0>();
+    case 7: return shape_of<F2>();
+    case 8: return shape_of<F3>();
     default: return shape_of<V0>();
     }
 }
@@ -849,7 +1091,19 @@ long long active_items(const BpJob& J, int variant, int zgs) {
 
 }  // namespace
 
-int bp_default_variant(int n_out, int nz, int sms) {
+int bp_default_variant(int n_out, int nz, int na, int sms) {
+    // Few angles: the kernel without columns (few_tile), up to where the columns are
+    // as fast, which for launches that do not fill the SMs is later, a call being mostly
+    // one tile's serial chain there. us per FBP, columns / without, at 512^2 x 64: 116.5
+    // / 115.9 with 24 angles, 129.8 / 144.0 with 32; 512^2 x 8: 38.7 / 32.1 with 32, 42.7
+    // / 42.2 with 48; 512^2 x 4, which has no pairs: 33.9 / 31.8 with 48; 64^2 x 8: 16.9
+    // / 14.6 with 64, 17.4 / 17.0 with 80.
+    const long long ctas = static_cast<long long>((n_out + 31) / 32) * ((n_out + 31) / 32) * ((nz + 3) / 4);
+    if (na <= (ctas <= sms || (ctas <= 4 * sms && nz <= 4) ? 64 : ctas <= 4 * sms ? 40 : 24)) {
+        // 32x32 once its CTAs reach the SM count, 32x16 above a quarter of it (64^2 x 16
+        // x 101: 16x16 25 us, 32x16 31, 32x32 44)
+        return ctas >= sms ? 6 : 4 * ctas >= sms ? 7 : 8;
+    }
     // The shape whose launch is estimated fastest for the job alone; a smaller
     // tile has to gain 15 % in the estimate, which leaves its own start-up cost
     // out. Measured on B200, us per FBP, 32x32 / 32x16 / 16x16: 27.8 / 21.7 / 19.7
@@ -883,7 +1137,7 @@ void bp_number_items(BpBatch& b, int variant, int sms) {
         one += active_items(b.job[k], variant, 1);
         two += active_items(b.job[k], variant, 2);
     }
-    const bool pair = variant != 1 && launch_cost(variant, 2, two, sms) < launch_cost(variant, 1, one, sms);
+    const bool pair = variant != 1 && variant < kBpVariants && launch_cost(variant, 2, two, sms) < launch_cost(variant, 1, one, sms);
     b.total = 0;
     for (int k = 0; k < b.njobs; ++k) {
         BpJob& J = b.job[k];
@@ -956,6 +1210,9 @@ cudaError_t launch_backproject_batch(const BpBatch& b, int variant, unsigned* d_
     case 3: return launch_many<V3>(b, persistent, d_counter, d_err, st);
     case 4: return launch_many<V4>(b, persistent, d_counter, d_err, st);
     case 5: return launch_many<V5>(b, persistent, d_counter, d_err, st);
+    case 6: return launch_many<F0>(b, persistent, d_counter, d_err, st);
+    case 7: return launch_many<F2>(b, persistent, d_counter, d_err, st);
+    case 8: return launch_many<F3>(b, persistent, d_counter, d_err, st);
     default: return launch_many<V0>(b, persistent, d_counter, d_err, st);
     }
 }
@@ -978,6 +1235,9 @@ cudaError_t launch_backproject(const float4* d_filt, int nz, int na, const FiltL
     case 3: return launch_one<V3>(b, d_err, st);
     case 4: return launch_one<V4>(b, d_err, st);
     case 5: return launch_one<V5>(b, d_err, st);
+    case 6: return launch_one<F0>(b, d_err, st);
+    case 7: return launch_one<F2>(b, d_err, st);
+    case 8: return launch_one<F3>(b, d_err, st);
     default: return launch_one<V0>(b, d_err, st);
     }
 }

@@ -146,11 +146,12 @@ std::vector<int> bp_bucket(int n_out, int nz, int na) {
 
 int bp_variant_for(const ctb_ctx* ctx, int n_out, int nz, int na) {
     if (ctx->bp_variant >= 0) return ctx->bp_variant;
-    if (ctx->autotune) {
+    const int variant = bp_default_variant(n_out, nz, na, ctx->sms);
+    if (ctx->autotune && variant < kBpVariants) {
         auto it = ctx->tuned.find(bp_bucket(n_out, nz, na));
         if (it != ctx->tuned.end()) return it->second;
     }
-    return bp_default_variant(n_out, nz, ctx->sms);
+    return variant;
 }
 
 ctb_status check_error_word(ctb_ctx* ctx) {
@@ -380,7 +381,7 @@ ctb_status fbp_stage(ctb_ctx* ctx, const float* d_sino, int nz, int na, int bins
     mark(ctx, ev, 3);
     const int zs = shape_depth > 0 ? shape_depth : nz;
     int variant = bp_variant_for(ctx, n_out, zs, na);
-    if (ctx->autotune && ctx->bp_variant < 0 && !ctx->tuned.count(bp_bucket(n_out, zs, na)))
+    if (ctx->autotune && ctx->bp_variant < 0 && variant < kBpVariants && !ctx->tuned.count(bp_bucket(n_out, zs, na)))
         CTB_TRY(tune_backprojection(ctx, d_filt, nz, na, fl, n_out, trig, d_stats, denorm, d_out, &variant, zs));
     CTB_LAUNCH(ctx, launch_backproject(d_filt, nz, na, fl, n_out, trig, d_stats, denorm, d_out,
                                        ctx->d_err, ctx->stream, variant, ctx->convention,
@@ -691,7 +692,7 @@ ctb_status ctb_bp_shape_info(int variant, int* tile_x, int* tile_y, int* voxels_
 ctb_status ctb_bp_shape_for(ctb_ctx* ctx, int output_size, int depth, int num_angles, int* variant) {
     if (!ctx || !variant || output_size <= 0 || depth <= 0 || num_angles <= 0) return CTB_ERR_INVALID;
     Guard g(ctx);
-    *variant = bp_variant_for(ctx, output_size, depth, num_angles);
+    *variant = bp_public_variant(bp_variant_for(ctx, output_size, depth, num_angles));
     return CTB_OK;
 }
 

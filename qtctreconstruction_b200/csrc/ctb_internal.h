@@ -57,8 +57,13 @@ struct BpShape {
     int tx, ty, vpt, ca, win;
 };
 BpShape bp_shape(int variant);
-// The shape used without tuning: a function of the job's size only.
-int bp_default_variant(int n_out, int nz, int sms);
+// The shape used without tuning: a function of the job's size only. From kBpVariants
+// on, the shapes of the kernel for few angles, which are neither tuned nor forced:
+// 32x32, 32x16, 16x16, the tiles of shapes 0, 2 and 3.
+int bp_default_variant(int n_out, int nz, int na, int sms);
+inline int bp_public_variant(int variant) {
+    return variant < kBpVariants ? variant : variant == kBpVariants ? 0 : variant - kBpVariants + 1;
+}
 
 // FilterDesign (FilterDesign.cpp:13-111) in double precision: fft_size/2+1 values.
 std::vector<double> filter_response(int L, int type);

@@ -133,9 +133,13 @@ extern "C" ctb_status ctb_fbp_noalloc(const float* d_sino, int depth, int num_an
     if (e == cudaSuccess)
         e = launch_filter(d_sino, depth, num_angles, g, fl, d_Hc, d_tw, nullptr, CTB_DENORM_NONE, scale,
                           d_filt, st);
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int variant = bp_default_variant(output_size, depth, num_angles, sms);
     if (e == cudaSuccess)
         e = launch_backproject(d_filt, depth, num_angles, fl, output_size, trig, nullptr,
-                               CTB_DENORM_NONE, d_out, d_err, st);
+                               CTB_DENORM_NONE, d_out, d_err, st, variant < kBpVariants ? 0 : variant);
     // the host vectors above must outlive the queued copies, and a bounded
     // device wait that gave up is reported through the error word
     unsigned h_err = 0;

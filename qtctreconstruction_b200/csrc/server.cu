@@ -379,7 +379,7 @@ ctb_status launch_batch(ctb_server* s, const std::vector<SReq*>& reqs, int slot)
     // request, a function of its size), one CTA per (request, slice group,
     // tile) item, most angles first
     std::vector<int> var(n);
-    for (int k = 0; k < n; ++k) var[k] = bp_default_variant(reqs[k]->r.output_size, reqs[k]->r.depth, s->sms);
+    for (int k = 0; k < n; ++k) var[k] = bp_default_variant(reqs[k]->r.output_size, reqs[k]->r.depth, reqs[k]->r.num_angles, s->sms);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
         return var[a] != var[b] ? var[a] < var[b] : reqs[a]->r.num_angles > reqs[b]->r.num_angles;
