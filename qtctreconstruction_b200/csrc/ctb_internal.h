@@ -112,9 +112,13 @@ inline Trig trig_view(void* table, int na, void* order = nullptr) {
 
 // Launch of a kernel that may start while the kernel before it in the stream
 // ends (programmatic dependent launch). Such a kernel calls chain_wait before it
-// reads or writes global memory: from there on every earlier kernel of the stream
-// is complete and its writes are visible. chain_wait then lets the next kernel's
-// blocks start, once all of this kernel's have. Measured, us per call: 23.6 -> 19.0
+// writes global memory or reads any that a kernel of the stream may write (tables
+// whose upload the host waited for may be read earlier): from there on every earlier
+// kernel of the stream is complete and its writes are visible. chain_wait then lets
+// the next kernel's blocks start, once all of this kernel's have. What the kernel
+// before may have written is read by ld_chained, never through the read-only path
+// (__ldg, or const __restrict__ parameters): that path asks for data which nothing
+// writes while the kernel runs, and this one is running while they are written. Measured, us per call: 23.6 -> 19.0
 // for an FBP of 64^2 x 16 x 101, 415 -> 404 for a forward projection of 300^2 x 37 x
 // 450, 32.8 -> 27.2 of 160^2 x 1 x 180.
 template <typename... P, typename... A>
@@ -136,6 +140,22 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, s
 __device__ __forceinline__ void chain_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// Loads that stay behind chain_wait (volatile) and do not use the read-only path.
+__device__ __forceinline__ float ld_chained(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_chained(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ int2 ld_chained(const int2* p) {
+    int2 v;
+    asm volatile("ld.global.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
 }
 #endif
 

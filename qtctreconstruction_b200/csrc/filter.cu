@@ -326,7 +326,7 @@ __device__ __forceinline__ void first_pass(float2* buf, int L, int tid, int T, c
         for (int r = 0; r < R / 2; ++r) {
             const int i = j + r * LR;
             const bool in = i < nd;
-            v[bi][r] = make_float2(in && r0 ? __ldg(r0 + i) : 0.0f, in && r1 ? __ldg(r1 + i) : 0.0f);
+            v[bi][r] = make_float2(in && r0 ? ld_chained(r0 + i) : 0.0f, in && r1 ? ld_chained(r1 + i) : 0.0f);
         }
         dft_half<R, false>(v[bi]);
     }
@@ -758,8 +758,8 @@ __global__ void __launch_bounds__(filter4_threads(LOGL), filter4_resident(LOGL) 
             for (int r = 0; r < R0 / 2; ++r) {
                 const int i = j + r * LR;
                 const bool in = i < nd;
-                v[r].re = make_float2(in && rows[0] ? __ldg(rows[0] + i) : 0.0f, in && rows[2] ? __ldg(rows[2] + i) : 0.0f);
-                v[r].im = make_float2(in && rows[1] ? __ldg(rows[1] + i) : 0.0f, in && rows[3] ? __ldg(rows[3] + i) : 0.0f);
+                v[r].re = make_float2(in && rows[0] ? ld_chained(rows[0] + i) : 0.0f, in && rows[2] ? ld_chained(rows[2] + i) : 0.0f);
+                v[r].im = make_float2(in && rows[1] ? ld_chained(rows[1] + i) : 0.0f, in && rows[3] ? ld_chained(rows[3] + i) : 0.0f);
             }
             dftp<R0, false, true>(v);
 #pragma unroll

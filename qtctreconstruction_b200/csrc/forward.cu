@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(1024) k_bp_order(const double2* __restrict__ c
 // stats[z] = {min, max, span_fwd, span_denorm} (SerialBackend.cpp:70-80, 298-300).
 // With box set, also empties the non-zero bounding box of each 4-slice group
 // that k_normalize then fills.
-__global__ void __launch_bounds__(1024) k_slice_stats(const float* __restrict__ vol, long long npx,
+__global__ void __launch_bounds__(1024) k_slice_stats(const float* vol, long long npx,
                                                       float4* __restrict__ stats, int4* __restrict__ box,
                                                       int2* __restrict__ band, int nband) {
     const int z = blockIdx.x;
@@ -100,13 +100,13 @@ __global__ void __launch_bounds__(1024) k_slice_stats(const float* __restrict__ 
     if ((npx & 3) == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
         const float4* p4 = reinterpret_cast<const float4*>(p);
         for (long long i = threadIdx.x; i < npx / 4; i += blockDim.x) {
-            const float4 v = __ldg(p4 + i);
+            const float4 v = ld_chained(p4 + i);
             lo = fminf(lo, fminf(fminf(v.x, v.y), fminf(v.z, v.w)));
             hi = fmaxf(hi, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
         }
     } else {
         for (long long i = threadIdx.x; i < npx; i += blockDim.x) {
-            const float v = __ldg(p + i);
+            const float v = ld_chained(p + i);
             lo = fminf(lo, v);
             hi = fmaxf(hi, v);
         }
@@ -154,8 +154,9 @@ __global__ void __launch_bounds__(1024) k_slice_stats(const float* __restrict__ 
 // each) get the x range of their non-zero pixels, followed by its ceil(w/8)
 // column bands with their y range (emptied by k_slice_stats too). With single, the
 // copies of a one-slice stack are planes of 4-byte pixels in the same layout.
+// (vol is older than k_slice_stats, which runs between: the read-only path may be used.)
 __global__ void __launch_bounds__(256) k_normalize(const float* __restrict__ vol, int w, int h, int nz,
-                                                   const float4* __restrict__ stats,
+                                                   const float4* stats,
                                                    float4* __restrict__ img, float4* __restrict__ imgT,
                                                    int skip_zero, int4* __restrict__ box,
                                                    int2* __restrict__ band, int single) {
@@ -304,7 +305,7 @@ __global__ void __launch_bounds__(256) k_normalize(const float* __restrict__ vol
 // -1 < x < w, -1 < y < h in double and widened by one sample each side. Pixel
 // columns read lie in [-2, w + 1] (inside the zero border); rows above the
 // image are skipped explicitly, rows below it are the zero rows of the plane.
-__global__ void __launch_bounds__(128) k_raymarch(const float4* __restrict__ img, int w, int h, int nz, int na,
+__global__ void __launch_bounds__(128) k_raymarch(const float4* img, int w, int h, int nz, int na,
                                                   int nd, float det_center, const double2* __restrict__ cs,
                                                   float* __restrict__ sino) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;

@@ -84,12 +84,13 @@ struct FAngle {
 };
 
 __device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
-// One pixel of a plane pair: 8 slices in 32 bytes (32-byte aligned), one load.
+// One pixel of a plane pair: 8 slices in 32 bytes (32-byte aligned), one load
+// (ld_chained: the normalisation before this kernel may still run when it starts).
 __device__ __forceinline__ void ld_pixel(const float4* p, float4 (&v)[NP]) {
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[0].z), "=f"(v[0].w), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[1].z),
-          "=f"(v[1].w)
-        : "l"(p));
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[0].z), "=f"(v[0].w), "=f"(v[1].x), "=f"(v[1].y),
+                   "=f"(v[1].z), "=f"(v[1].w)
+                 : "l"(p));
 }
 __device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
 
@@ -108,7 +109,7 @@ struct RowRec {
 // Eight rows of a block. Lane l's pixel of a row lies y = cl1 + dy bins from bin
 // m_l + 1 (cl1 = l |kq| - m_l - 1), y in [-1, 1], which gives its hat weights
 // for bins m_l, m_l + 1, m_l + 2: max(-y, 0), 1 - |y|, max(y, 0).
-__device__ __forceinline__ void walk_rows(const float4* __restrict__ lane_base, const RowRec* __restrict__ rr,
+__device__ __forceinline__ void walk_rows(const float4* lane_base, const RowRec* __restrict__ rr,
                                           float cl1, float2 (&acc)[3][2 * NP]) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -131,11 +132,11 @@ __device__ __forceinline__ void walk_rows(const float4* __restrict__ lane_base, 
 
 // The same for a single slice (4-byte pixels), two rows at a time: the two lanes
 // of a packed operation hold an even and an odd row, so the weights need no copies.
-__device__ __forceinline__ void walk_rows(const float* __restrict__ lane_base, const RowRec* __restrict__ rr, float cl1,
+__device__ __forceinline__ void walk_rows(const float* lane_base, const RowRec* __restrict__ rr, float cl1,
                                           float2 (&acc)[3]) {
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {
-        const float2 v = make_float2(__ldg(lane_base + rr[i].col), __ldg(lane_base + rr[i + 1].col));
+        const float2 v = make_float2(ld_chained(lane_base + rr[i].col), ld_chained(lane_base + rr[i + 1].col));
         const float2 y = make_float2(cl1 + rr[i].dy, cl1 + rr[i + 1].dy);
         acc[0] = __ffma2_rn(make_float2(fmaxf(-y.x, 0.0f), fmaxf(-y.y, 0.0f)), v, acc[0]);
         acc[1] = __ffma2_rn(make_float2(1.0f - fabsf(y.x), 1.0f - fabsf(y.y)), v, acc[1]);
@@ -151,7 +152,7 @@ __device__ __forceinline__ void walk_rows(const float* __restrict__ lane_base, c
 // [0, 1] (bin 0) or [nd-2, nd] (bin nd-1), the reference's float s being
 // much closer than that to the exact one. The lanes' sums are added by a
 // fixed shuffle tree; every lane returns the total.
-__device__ __noinline__ void edge_bin(const float4* __restrict__ plane, int pitch, int nq,
+__device__ __noinline__ void edge_bin(const float4* plane, int pitch, int nq,
                                       const FAngle& f, int b_lo, int e, int nd, int r_lo, int r_hi, bool rows,
                                       float cxf, float cyf, int lane, float2 (&sum)[2 * NP]) {
 #pragma unroll
@@ -179,7 +180,7 @@ __device__ __noinline__ void edge_bin(const float4* __restrict__ plane, int pitc
             const float4* px = plane + 2 * (static_cast<long long>(p) * pitch + c);
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
-                const float4 v = __ldg(px + k);
+                const float4 v = ld_chained(px + k);
                 sum[2 * k] = __ffma2_rn(W, lo2(v), sum[2 * k]);
                 sum[2 * k + 1] = __ffma2_rn(W, hi2(v), sum[2 * k + 1]);
             }
@@ -194,7 +195,7 @@ __device__ __noinline__ void edge_bin(const float4* __restrict__ plane, int pitc
 }
 
 // edge_bin of a single slice.
-__device__ __noinline__ float edge_bin(const float* __restrict__ plane, int pitch, int nq, const FAngle& f, int b_lo, int e,
+__device__ __noinline__ float edge_bin(const float* plane, int pitch, int nq, const FAngle& f, int b_lo, int e,
                                        int nd, int r_lo, int r_hi, bool rows, float cxf, float cyf, int lane) {
     float sum = 0.0f;
     const double lo = e == 0 ? 0.0 : nd - 2.0, hi = e == 0 ? 1.0 : static_cast<double>(nd);
@@ -210,7 +211,7 @@ __device__ __noinline__ float edge_bin(const float* __restrict__ plane, int pitc
         for (int i = 0; i < 3; ++i) {
             const int c = c0 + i;
             const bool in = c >= 0 && c <= c1;
-            v[i] = __ldg(plane + static_cast<long long>(p) * pitch + (in ? c : 0));
+            v[i] = ld_chained(plane + static_cast<long long>(p) * pitch + (in ? c : 0));
             const float xg = static_cast<float>(rows ? c : p);
             const float yg = static_cast<float>(rows ? p : c);
             const float ss = __fadd_rn(__fadd_rn(__fmul_rn(__fsub_rn(xg, cxf), f.cf),
@@ -243,14 +244,14 @@ constexpr int FULL = 7, SPARSE = 4;
 // 34.6 at 256^2 x 360, 348 -> 154 at 512^2 x 720, 2336 -> 991 at 1024^2 x 1440).
 template <int PER_SM, bool ONE>
 __global__ void __launch_bounds__(THREADS, PER_SM)
-    k_forward(const float4* __restrict__ img, const float4* __restrict__ imgT, int w, int h, int nz, int na, int nd,
-              const int4* __restrict__ groups, const FwdAngleRec* __restrict__ arec, const int4* __restrict__ box,
-              const int2* __restrict__ band, float* __restrict__ sino) {
+    k_forward(const float4* img, const float4* imgT, int w, int h, int nz, int na, int nd,
+              const int4* __restrict__ groups, const FwdAngleRec* __restrict__ arec, const int4* box,
+              const int2* band, float* __restrict__ sino) {
     __shared__ FAngle fa[GMAX];
     __shared__ int erow[GMAX][4];                      // edge-pass rows: bin 0 [lo, hi], bin nd-1 [lo, hi]
     __shared__ __align__(16) RowRec rows_sm[GMAX][LANES];  // the block of rows each warp walks
 
-    const int4 grp = groups[blockIdx.y];
+    const int4 grp = groups[blockIdx.y];  // the plan: its upload was waited for
     const int cnt = grp.y;
     const bool rows = grp.z == 0;
     const int K = grp.w;  // output bins per strip for this group
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__(THREADS, PER_SM)
                 const int bi = p >> 3;
                 for (int k = 0; k < NP && bi < nb_p; ++k) {
                     if (g0 + k >= ng4) break;
-                    const int2 r = __ldg(band + static_cast<long long>(g0 + k) * nb_all + nb_off + bi);
+                    const int2 r = ld_chained(band + static_cast<long long>(g0 + k) * nb_all + nb_off + bi);
                     cl = min(cl, r.x);
                     ch = max(ch, r.y);
                 }
