@@ -657,26 +657,33 @@ template <class C>
 struct FewSmem {
     float4 win[2][C::CA][C::WIN];
     FewRec rec[2][C::CA];
-    unsigned long long bar[2];
 };
 template <class C>
 using SmemOf = std::conditional_t<C::FEW, FewSmem<C>, BpSmem<C>>;
-
+// The shape of a launch's jobs of few angles: the same tiles, in the windows' space.
 template <class C>
-__device__ __forceinline__ void bp_init(FewSmem<C>& S) {
-    if (threadIdx.x == 0) {
-        for (int b = 0; b < 2; ++b) mbar_init(&S.bar[b], 1);
-        mbar_fence_init();
-    }
-}
+struct FewOf {
+    static constexpr bool ANY = false;
+    using type = F0;
+};
+template <class F, class C>
+struct FewIn {
+    static constexpr bool ANY = true;
+    using type = F;
+    static_assert(F::TX == C::TX && F::TY == C::TY, "one grid of tiles for both");
+    static_assert(sizeof(FewSmem<F>) <= sizeof(BpSmem<C>::win), "clear of the barriers");
+};
+template <> struct FewOf<V0> : FewIn<F0, V0> {};
+template <> struct FewOf<V2> : FewIn<F2, V2> {};
+template <> struct FewOf<V3> : FewIn<F3, V3> {};
 
-// Backproject one tile (x0, y0) of slice group zg of job J. `chunks` counts the
+// Backproject one tile (x0, y0) of slice group zg of job J. bar: one per buffer. `chunks` counts the
 // chunks this CTA has consumed so far (mbarrier phases continue across items).
 // Returns false when a bounded wait gave up (block-uniform), the copies under way
 // waited for.
 template <class C>
-__device__ __forceinline__ bool few_tile(FewSmem<C>& S, const BpJob& J, int zg, int x0, int y0, unsigned& chunks,
-                                         unsigned* err) {
+__device__ __forceinline__ bool few_tile(FewSmem<C>& S, unsigned long long* bar, const BpJob& J, int zg, int x0, int y0,
+                                         unsigned& chunks, unsigned* err) {
     constexpr int TX = C::TX, TY = C::TY, VPT = C::VPT, XS = C::XS, CA = C::CA, WIN = C::WIN;
     const int t = threadIdx.x;
     const int lx = t % XS, ly = t / XS;
@@ -748,9 +755,9 @@ __device__ __forceinline__ bool few_tile(FewSmem<C>& S, const BpJob& J, int zg, 
             r.pad[0] = r.pad[1] = 0;
             S.rec[b][t] = r;
             bulk_load(&S.win[b][t][0], plane + static_cast<long long>(a) * J.pitch + J.guard + ws,
-                      WIN * sizeof(float4), &S.bar[b]);
+                      WIN * sizeof(float4), &bar[b]);
         }
-        if (t == 0) mbar_expect_tx(&S.bar[b], static_cast<unsigned>(cnt * WIN * sizeof(float4)));
+        if (t == 0) mbar_expect_tx(&bar[b], static_cast<unsigned>(cnt * WIN * sizeof(float4)));
     };
 
     float4 acc[VPT];
@@ -778,7 +785,7 @@ __device__ __forceinline__ bool few_tile(FewSmem<C>& S, const BpJob& J, int zg, 
         if (c + 1 < nch) issue(c + 1, (g + 1) & 1);
         // A failed wait leaves stale window data; the block then stops as a
         // whole at the barrier below (the decision is block-uniform).
-        const bool landed = mbar_wait_bounded(&S.bar[b], (g >> 1) & 1, err);
+        const bool landed = mbar_wait_bounded(&bar[b], (g >> 1) & 1, err);
         const int cnt = min(CA, na - c * CA);
         for (int j = 0; j < cnt; ++j) {
             const FewRec r = S.rec[b][j];
@@ -833,8 +840,8 @@ __device__ __forceinline__ bool few_tile(FewSmem<C>& S, const BpJob& J, int zg, 
         }
         if (!__syncthreads_and(landed)) {
             if (t == 0) {
-                mbar_wait_bounded(&S.bar[b], (g >> 1) & 1, err);
-                if (c + 1 < nch) mbar_wait_bounded(&S.bar[b ^ 1], ((g + 1) >> 1) & 1, err);
+                mbar_wait_bounded(&bar[b], (g >> 1) & 1, err);
+                if (c + 1 < nch) mbar_wait_bounded(&bar[b ^ 1], ((g + 1) >> 1) & 1, err);
             }
             __syncthreads();
             return false;
@@ -860,11 +867,6 @@ __device__ __forceinline__ bool few_tile(FewSmem<C>& S, const BpJob& J, int zg, 
 
 // One item: the tile (x0, y0) of slice groups zg J.zgs ... of job J (a pair, or
 // one group where a pair would pass the last slice).
-template <class C>
-__device__ __forceinline__ bool bp_item(FewSmem<C>& S, const BpJob& J, int zg, int x0, int y0, unsigned& chunks,
-                                        unsigned* err) {
-    return few_tile<C>(S, J, zg, x0, y0, chunks, err);
-}
 template <class C>
 __device__ __forceinline__ bool bp_item(BpSmem<C>& S, const BpJob& J, int zi, int x0, int y0, unsigned& stages,
                                         unsigned* err) {
@@ -896,27 +898,41 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
                                                                   unsigned* __restrict__ counter,
                                                                   unsigned* __restrict__ err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    SmemOf<C>& S = *reinterpret_cast<SmemOf<C>*>(smem_raw);
     __shared__ int s_item;
-    bp_init(S);
+    __shared__ unsigned long long few_bar[2];
+    constexpr bool MIX = MODE != 0 && FewOf<C>::ANY;  // jobs of few angles among the others
+    if constexpr (C::FEW || MIX) {
+        if (threadIdx.x == 0)
+            for (int b = 0; b < 2; ++b) mbar_init(&few_bar[b], 1);
+    }
+    if constexpr (!C::FEW) bp_init(*reinterpret_cast<BpSmem<C>*>(smem_raw));
+    else if (threadIdx.x == 0) mbar_fence_init();
     chain_wait();  // lets the next call's first kernel start in this one's tail
-    unsigned stages = 0;
+    unsigned stages = 0, chunks = 0;
+    // item `local` of job J
+    auto run = [&](const BpJob& J, int local) {
+        const int zi = local / J.tiles, tl = local - zi * J.tiles;
+        const int x0 = (tl % J.tiles_x) * C::TX, y0 = (tl / J.tiles_x) * C::TY;
+        if constexpr (C::FEW) {
+            return few_tile<C>(*reinterpret_cast<FewSmem<C>*>(smem_raw), few_bar, J, zi, x0, y0, chunks, err);
+        } else {
+            if constexpr (MIX) {
+                using F = typename FewOf<C>::type;
+                if (J.few)
+                    return few_tile<F>(*reinterpret_cast<FewSmem<F>*>(smem_raw), few_bar, J, zi, x0, y0, chunks, err);
+            }
+            return bp_item(*reinterpret_cast<BpSmem<C>*>(smem_raw), J, zi, x0, y0, stages, err);
+        }
+    };
     if constexpr (MODE == 0) {
         __syncthreads();
-        const BpJob& J = batch.job[0];
-        const int zg = blockIdx.x / J.tiles;
-        const int tl = blockIdx.x - zg * J.tiles;
-        bp_item(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, stages, err);
+        run(batch.job[0], blockIdx.x);
     } else if constexpr (MODE == 1) {
         __syncthreads();
         const int item = blockIdx.x;
         int j = 0;
         while (j + 1 < batch.njobs && batch.job[j + 1].first <= item) ++j;
-        const BpJob& J = batch.job[j];
-        const int local = item - static_cast<int>(J.first);
-        const int zg = local / J.tiles;
-        const int tl = local - zg * J.tiles;
-        bp_item(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, stages, err);
+        run(batch.job[j], item - static_cast<int>(batch.job[j].first));
     } else {
         for (;;) {
             if (threadIdx.x == 0) s_item = static_cast<int>(atomicAdd(counter, 1u));
@@ -925,12 +941,11 @@ __global__ void __launch_bounds__(THREADS, C::MINB) k_backproject(const __grid_c
             if (item >= batch.total) break;
             int j = 0;
             while (j + 1 < batch.njobs && batch.job[j + 1].first <= item) ++j;
-            const BpJob& J = batch.job[j];
-            const int local = item - static_cast<int>(J.first);
-            const int zg = local / J.tiles;
-            const int tl = local - zg * J.tiles;
-            if (!bp_item(S, J, zg, (tl % J.tiles_x) * C::TX, (tl / J.tiles_x) * C::TY, stages, err)) break;
-            __syncthreads();  // shared state of this item is dead before the next item's staging
+            if (!run(batch.job[j], item - static_cast<int>(batch.job[j].first))) break;
+            // shared state of this item is dead before the next item's staging, also
+            // where one kind's copies land in the other's records
+            if constexpr (MIX) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
         }
     }
 }
@@ -1135,13 +1150,13 @@ void bp_number_items(BpBatch& b, int variant, int sms) {
     long long one = 0, two = 0;
     for (int k = 0; k < b.njobs; ++k) {
         one += active_items(b.job[k], variant, 1);
-        two += active_items(b.job[k], variant, 2);
+        two += active_items(b.job[k], variant, b.job[k].few ? 1 : 2);
     }
-    const bool pair = variant != 1 && variant < kBpVariants && launch_cost(variant, 2, two, sms) < launch_cost(variant, 1, one, sms);
+    const bool pair = variant != 1 && launch_cost(variant, 2, two, sms) < launch_cost(variant, 1, one, sms);
     b.total = 0;
     for (int k = 0; k < b.njobs; ++k) {
         BpJob& J = b.job[k];
-        J.zgs = pair ? 2 : 1;
+        J.zgs = pair && !J.few ? 2 : 1;
         J.first = b.total;
         b.total += static_cast<long long>(J.tiles) * (((J.nz + 3) / 4 + J.zgs - 1) / J.zgs);
     }
@@ -1197,6 +1212,7 @@ BpJob make_bp_job(const float4* d_filt, int nz, int na, const FiltLayout& fl, in
     J.tiles = J.tiles_x * ((n_out + sh.ty - 1) / sh.ty);
     J.first = 0;
     J.zgs = 1;
+    J.few = variant >= kBpVariants;
     return J;
 }
 
@@ -1204,15 +1220,19 @@ cudaError_t launch_backproject_batch(const BpBatch& b, int variant, unsigned* d_
                                      cudaStream_t st, bool persistent) {
     if (b.total == 0) return cudaSuccess;
     if (b.total > 0x7fffffffLL) return cudaErrorInvalidValue;
+    bool all_few = true;  // four CTAs per SM instead of the columns' three
+    for (int k = 0; k < b.njobs; ++k) all_few = all_few && b.job[k].few;
+    if (all_few) {
+        if (variant == 0) return launch_many<F0>(b, persistent, d_counter, d_err, st);
+        if (variant == 2) return launch_many<F2>(b, persistent, d_counter, d_err, st);
+        return launch_many<F3>(b, persistent, d_counter, d_err, st);
+    }
     switch (variant) {
     case 1: return launch_many<V1>(b, persistent, d_counter, d_err, st);
     case 2: return launch_many<V2>(b, persistent, d_counter, d_err, st);
     case 3: return launch_many<V3>(b, persistent, d_counter, d_err, st);
     case 4: return launch_many<V4>(b, persistent, d_counter, d_err, st);
     case 5: return launch_many<V5>(b, persistent, d_counter, d_err, st);
-    case 6: return launch_many<F0>(b, persistent, d_counter, d_err, st);
-    case 7: return launch_many<F2>(b, persistent, d_counter, d_err, st);
-    case 8: return launch_many<F3>(b, persistent, d_counter, d_err, st);
     default: return launch_many<V0>(b, persistent, d_counter, d_err, st);
     }
 }

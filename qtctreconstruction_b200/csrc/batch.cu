@@ -160,24 +160,25 @@ ctb_status build(ctb_batch* b) {
         }
         b->filt.push_back(f);
     }
-    // backprojection: one persistent launch per tile shape, most angles first
-    // (the most expensive items lead the queue)
+    // backprojection: one launch per tile shape, most angles first (the most
+    // expensive items lead the queue)
     std::vector<int> by_na(n);
     std::iota(by_na.begin(), by_na.end(), 0);
     std::stable_sort(by_na.begin(), by_na.end(), [&](int x, int y) {
-        return var[x] != var[y] ? var[x] < var[y] : b->jobs[x].num_angles > b->jobs[y].num_angles;
+        const int vx = bp_public_variant(var[x]), vy = bp_public_variant(var[y]);
+        return vx != vy ? vx < vy : b->jobs[x].num_angles > b->jobs[y].num_angles;
     });
     if (per_job) std::iota(by_na.begin(), by_na.end(), 0);
     for (int k = 0; k < n;) {
         BpBatch p;
-        const int v = var[by_na[k]];
-        while (k < n && p.njobs < cap && var[by_na[k]] == v) {
+        const int own = var[by_na[k]], v = bp_public_variant(own);
+        while (k < n && p.njobs < cap && bp_public_variant(var[by_na[k]]) == v) {
             p.job[p.njobs++] = bj[by_na[k]];
             ++k;
         }
         bp_number_items(p, v, ctx->sms);
         b->bp.push_back(p);
-        b->bp_variant.push_back(v);
+        b->bp_variant.push_back(per_job ? own : v);
     }
     b->kernel_launches = static_cast<int>(b->filt.size() + b->bp.size());
 

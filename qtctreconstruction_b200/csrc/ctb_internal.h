@@ -287,6 +287,7 @@ struct BpJob {
     int edge_rule;        // 1: SerialBackend's tap rule (both taps in range); 0: per-tap bounds
     int tiles_x, tiles;   // tiles per row / per slice group
     int zgs;              // slice groups per item (1 or 2)
+    int few;              // few angles: no columns (always one slice group per item)
     long long first;      // index of the job's first item in the batch
 };
 struct BpBatch {
@@ -327,7 +328,8 @@ FiltJob make_filt_job(const float* d_sino, int nz, int na, const PadGeom& g, con
 // Decide the slice groups per item of a batch (all of one tile shape) and number
 // its items: sets every job's zgs and first, and the total.
 void bp_number_items(BpBatch& b, int variant, int sms);
-// Backprojection of a batch (below 2^31 items, one tile shape): one CTA per
+// Backprojection of a batch (below 2^31 items, one tile shape: the variants of its jobs
+// have the same bp_public_variant, `variant`): one CTA per
 // item, or with `persistent` a grid of resident CTAs drawing items from
 // d_counter (zeroed here on the stream). Filtering takes one CTA per item.
 cudaError_t launch_backproject_batch(const BpBatch& b, int variant, unsigned* d_counter, unsigned* d_err,

@@ -379,19 +379,21 @@ ctb_status launch_batch(ctb_server* s, const std::vector<SReq*>& reqs, int slot)
     // request, a function of its size), one CTA per (request, slice group,
     // tile) item, most angles first
     std::vector<int> var(n);
-    for (int k = 0; k < n; ++k) var[k] = bp_default_variant(reqs[k]->r.output_size, reqs[k]->r.depth, reqs[k]->r.num_angles, s->sms);
+    for (int k = 0; k < n; ++k)
+        var[k] = bp_default_variant(reqs[k]->r.output_size, reqs[k]->r.depth, reqs[k]->r.num_angles, s->sms);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-        return var[a] != var[b] ? var[a] < var[b] : reqs[a]->r.num_angles > reqs[b]->r.num_angles;
+        const int va = bp_public_variant(var[a]), vb = bp_public_variant(var[b]);
+        return va != vb ? va < vb : reqs[a]->r.num_angles > reqs[b]->r.num_angles;
     });
     for (int k = 0; k < n;) {
         BpBatch bp;
-        const int v = var[order[k]];
-        while (k < n && bp.njobs < kMaxJobs && var[order[k]] == v) {
+        const int v = bp_public_variant(var[order[k]]);
+        while (k < n && bp.njobs < kMaxJobs && bp_public_variant(var[order[k]]) == v) {
             const SReq* q = reqs[order[k]];
             const Trig trig = trig_view(q->d_trig, q->r.num_angles, q->order.ptr);
             bp.job[bp.njobs++] = make_bp_job(q->d_filt, q->r.depth, q->r.num_angles, q->fl, q->r.output_size, trig, nullptr,
-                                             CTB_DENORM_NONE, q->d_out, v);
+                                             CTB_DENORM_NONE, q->d_out, var[order[k]]);
             ++k;
         }
         bp_number_items(bp, v, s->sms);

@@ -41,11 +41,12 @@ def test_parity(backend, n, bins, depth, na):
     _check(d_o.cpu().numpy(), sinos, n)
 
 
-@pytest.mark.parametrize("flags", [0, ctb.BATCH_GRAPH, ctb.BATCH_PERSISTENT])
+@pytest.mark.parametrize("flags", [0, ctb.BATCH_GRAPH, ctb.BATCH_PERSISTENT, ctb.BATCH_PER_JOB])
 def test_batches_equal_single_calls(backend, flags):
     import torch
     jobs, args = [], []
-    for n, depth, na in ((64, 5, 16), (64, 5, 120), (160, 33, 24), (160, 33, 30), (40, 9, 1), (300, 64, 24)):
+    for n, depth, na in ((64, 5, 16), (64, 5, 120), (128, 16, 60), (128, 16, 150), (160, 33, 24), (160, 33, 130), (40, 9, 1),
+                         (300, 64, 24)):
         bins = ctb.odd_detector_count(n)
         s = torch.from_numpy(np.random.default_rng(n + na).uniform(0.0, 1.0, (depth, na, bins)).astype(np.float32)).cuda()
         o, alone = (torch.full((depth, n, n), float("nan"), device="cuda") for _ in range(2))
