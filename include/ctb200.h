@@ -366,7 +366,9 @@ typedef struct ctb_server ctb_server;
 
 typedef struct ctb_server_config {
     int device;
-    size_t memory_budget;  /* device bytes for request state; 0 = min(120 GB, 85% of free) */
+    size_t memory_budget;  /* device bytes for request state; 0 = min(120 GB, 85% of free). Outside it:
+                              filter tables per size, and 2 MiB for the angle orders of admitted
+                              requests (a request also waits while they are full) */
     int max_batch;         /* requests per batch, 1..64; 0 = 64 */
     int copy_threads;      /* staging threads per direction; 0 = 4 */
     size_t staging_bytes;  /* pinned staging per copy thread; 0 = 64 MiB */

@@ -117,17 +117,17 @@ struct SReq {
     uint64_t seq = 0;
     ctb_request r{};
     std::vector<float> angles;
-    DevBuf order;            // the backprojector's angle order, a buffer of the server's pool
     State state = kPending;
     ctb_status status = CTB_ERR_BUSY;
     bool cancel = false;
     bool has_block = false;
-    size_t off = 0;
+    size_t off = 0, order_off = 0;
     size_t bytes = 0;
     size_t sino_bytes = 0, out_bytes = 0, trig_off = 0, filt_off = 0, sino_off = 0, out_off = 0;
     const float* d_sino = nullptr;
     float4* d_filt = nullptr;
     void* d_trig = nullptr;
+    void* d_order = nullptr;  // the backprojector's angle order
     float* d_out = nullptr;
     PadGeom g;
     FiltLayout fl;
@@ -149,6 +149,10 @@ struct Stager {
 constexpr int kMaxInflightBatches = 2;
 constexpr int kErrSlots = 8;
 constexpr int kMaxBypass = 16;  // times the oldest request may be overtaken by smaller ones
+// Angle orders of the admitted requests, beside the memory budget, which counts what
+// a request's own block holds: 15 requests of the most angles, 400 of 2560.
+constexpr size_t kOrderSpace = size_t(2) << 20;
+static_assert(kOrderSpace >= sizeof(int) * kBpGroups + sizeof(uint16_t) * kMaxAngles, "any request alone");
 
 }  // namespace
 
@@ -166,6 +170,8 @@ struct ctb_server {
     ctb_server_config cfg{};
     char* d_base = nullptr;
     ctb_arena arena;
+    char* d_orders = nullptr;
+    ctb_arena orders;
     cudaStream_t compute = nullptr;
     cudaStream_t table_stream = nullptr;
     int sms = 0;
@@ -180,7 +186,6 @@ struct ctb_server {
     std::mutex tables_mu;  // guards filters / twiddles (never held with mu)
     std::map<std::pair<int, int>, DevBuf> filters;
     std::map<int, DevBuf> twiddles;
-    std::vector<DevBuf> free_orders;  // angle-order buffers no request holds (guarded by mu)
     bool kick = false;     // something changed that may let a queued request in
     int inflight = 0;
     uint64_t batch_seq = 0;
@@ -227,10 +232,9 @@ void finalize(ctb_server* s, SReq* q, ctb_status st) {
     if (q->state == kFinal) return;
     if (q->has_block) {
         arena_free(&s->arena, q->off);
+        arena_free(&s->orders, q->order_off);
         q->has_block = false;
     }
-    if (q->order.ptr) s->free_orders.push_back(q->order);
-    q->order = DevBuf();
     q->state = kFinal;
     q->status = st;
     q->t_done = Clock::now();
@@ -251,11 +255,22 @@ void finalize(ctb_server* s, SReq* q, ctb_status st) {
 
 // Convolution spectrum and twiddles for a request (server cache; called at
 // submission with tables_mu held and mu not held: no CUDA call ever runs under
-// mu, which the batch callbacks take).
+// mu, which the batch callbacks take). The submitting thread may have any device
+// current; what is built here belongs to the server's.
 ctb_status request_tables(ctb_server* s, SReq* q) {
     const int Lc = q->g.Lc;
     auto key = std::make_pair(q->r.bins, q->r.filter);
     auto it = s->filters.find(key);
+    struct OnDevice {
+        int caller = -1;
+        ~OnDevice() {
+            if (caller >= 0) cudaSetDevice(caller);
+        }
+    } on_device;
+    if (it == s->filters.end() || !s->twiddles.count(Lc)) {
+        if (cudaGetDevice(&on_device.caller) != cudaSuccess || cudaSetDevice(s->cfg.device) != cudaSuccess)
+            return CTB_ERR_CUDA;
+    }
     if (it == s->filters.end()) {
         const std::vector<float2> Hc = filter_table(q->g, q->r.filter);
         DevBuf b;
@@ -286,34 +301,6 @@ ctb_status request_tables(ctb_server* s, SReq* q) {
     return CTB_OK;
 }
 
-// A device buffer for a request's angle order: one of the pool that is large
-// enough, else a new one (like the spectra, outside the memory budget; the pool
-// holds at most as many as requests were alive at once, and is freed with the
-// server). Called at submission, mu not held.
-ctb_status request_order(ctb_server* s, SReq* q) {
-    const size_t need = order_bytes(q->r.num_angles);
-    {
-        std::lock_guard<std::mutex> lk(s->mu);
-        for (DevBuf& b : s->free_orders)
-            if (b.bytes >= need) {
-                q->order = b;
-                b = s->free_orders.back();
-                s->free_orders.pop_back();
-                return CTB_OK;
-            }
-    }
-    size_t bytes = 8192;
-    while (bytes < need) bytes *= 2;
-    DevBuf b;
-    if (cudaMalloc(&b.ptr, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        return CTB_ERR_OOM;
-    }
-    b.bytes = bytes;
-    q->order = b;
-    return CTB_OK;
-}
-
 // Admit queued requests in arrival order while they fit (mu held). A request
 // that does not fit may be overtaken by smaller ones, the oldest such request
 // at most kMaxBypass times.
@@ -321,8 +308,13 @@ void admit(ctb_server* s) {
     SReq* blocked = nullptr;
     for (auto it = s->pending.begin(); it != s->pending.end();) {
         SReq* q = *it;
-        size_t off = 0;
-        if (!arena_alloc(&s->arena, q->bytes, &off)) {
+        size_t off = 0, order_off = 0;
+        bool fits = arena_alloc(&s->orders, order_bytes(q->r.num_angles), &order_off);
+        if (fits && !arena_alloc(&s->arena, q->bytes, &off)) {
+            arena_free(&s->orders, order_off);
+            fits = false;
+        }
+        if (!fits) {
             if (!blocked) {
                 blocked = q;
                 if (q->bypassed >= kMaxBypass) return;
@@ -333,9 +325,11 @@ void admit(ctb_server* s) {
         if (blocked) ++blocked->bypassed;
         it = s->pending.erase(it);
         q->off = off;
+        q->order_off = order_off;
         q->has_block = true;
         char* base = s->d_base + off;
         q->d_trig = base + q->trig_off;
+        q->d_order = s->d_orders + order_off;
         q->d_filt = reinterpret_cast<float4*>(base + q->filt_off);
         if (q->r.flags & CTB_REQ_DEVICE) {
             q->d_sino = q->r.sino;
@@ -391,7 +385,7 @@ ctb_status launch_batch(ctb_server* s, const std::vector<SReq*>& reqs, int slot)
         const int v = bp_public_variant(var[order[k]]);
         while (k < n && bp.njobs < kMaxJobs && bp_public_variant(var[order[k]]) == v) {
             const SReq* q = reqs[order[k]];
-            const Trig trig = trig_view(q->d_trig, q->r.num_angles, q->order.ptr);
+            const Trig trig = trig_view(q->d_trig, q->r.num_angles, q->d_order);
             bp.job[bp.njobs++] = make_bp_job(q->d_filt, q->r.depth, q->r.num_angles, q->fl, q->r.output_size, trig, nullptr,
                                              CTB_DENORM_NONE, q->d_out, var[order[k]]);
             ++k;
@@ -497,7 +491,7 @@ bool upload_trig(SReq* q, Stager& st) {
                cudaSuccess &&
            cudaMemcpyAsync(cs + na, csf.data(), sizeof(float2) * na, cudaMemcpyHostToDevice, st.stream) ==
                cudaSuccess &&
-           launch_trig(d_deg, na, trig_view(cs, na, q->order.ptr), st.stream) == cudaSuccess &&
+           launch_trig(d_deg, na, trig_view(cs, na, q->d_order), st.stream) == cudaSuccess &&
            cudaStreamSynchronize(st.stream) == cudaSuccess;
 }
 
@@ -649,8 +643,8 @@ void free_server(ctb_server* s) {
     for (auto& st : s->down_st) free_stager(st);
     for (auto& kv : s->filters) cudaFree(kv.second.ptr);
     for (auto& kv : s->twiddles) cudaFree(kv.second.ptr);
-    for (auto& b : s->free_orders) cudaFree(b.ptr);
     if (s->d_base) cudaFree(s->d_base);
+    if (s->d_orders) cudaFree(s->d_orders);
     if (s->d_err) cudaFree(s->d_err);
     if (s->h_err) cudaFreeHost(s->h_err);
     if (s->compute) cudaStreamDestroy(s->compute);
@@ -733,7 +727,8 @@ ctb_status ctb_server_create(const ctb_server_config* config, ctb_server** out) 
               cudaMalloc(&s->d_err, 2 * sizeof(unsigned)) == cudaSuccess &&
               cudaMemset(s->d_err, 0, 2 * sizeof(unsigned)) == cudaSuccess &&
               cudaHostAlloc(&s->h_err, kErrSlots * sizeof(unsigned), cudaHostAllocDefault) == cudaSuccess;
-    if (ok && cudaMalloc(&s->d_base, cfg.memory_budget) != cudaSuccess) {
+    if (ok && (cudaMalloc(&s->d_orders, kOrderSpace) != cudaSuccess ||
+               cudaMalloc(&s->d_base, cfg.memory_budget) != cudaSuccess)) {
         cudaGetLastError();
         free_server(s);
         delete s;
@@ -750,6 +745,7 @@ ctb_status ctb_server_create(const ctb_server_config* config, ctb_server** out) 
         return CTB_ERR_CUDA;
     }
     arena_init(&s->arena, cfg.memory_budget);
+    arena_init(&s->orders, kOrderSpace);
     s->sched = std::thread(scheduler, s);
     for (int i = 0; i < cfg.copy_threads; ++i) {
         s->up.emplace_back(uploader, s, i);
@@ -775,19 +771,12 @@ ctb_status ctb_server_submit(ctb_server* s, const ctb_request* req, uint64_t* id
     q->r.angles_deg = nullptr;
     plan_request(q.get());
     if (q->bytes <= s->arena.capacity) {  // capacity is fixed at creation
-        {
-            std::lock_guard<std::mutex> tl(s->tables_mu);
-            const ctb_status st = request_tables(s, q.get());
-            if (st != CTB_OK) return st;
-        }
-        const ctb_status st = request_order(s, q.get());
+        std::lock_guard<std::mutex> tl(s->tables_mu);
+        const ctb_status st = request_tables(s, q.get());
         if (st != CTB_OK) return st;
     }
     std::lock_guard<std::mutex> lk(s->mu);
-    if (s->stop) {
-        if (q->order.ptr) s->free_orders.push_back(q->order);
-        return CTB_ERR_CANCELLED;
-    }
+    if (s->stop) return CTB_ERR_CANCELLED;
     if (q->bytes > s->arena.capacity) {
         ++s->rejected;
         return CTB_ERR_OOM;
