@@ -389,59 +389,6 @@ ctb_status fbp_stage(ctb_ctx* ctx, const float* d_sino, int nz, int na, int bins
     return CTB_OK;
 }
 
-// Slabs of a host-buffer pipeline of slices with n_out x n_out voxels: {first
-// slice, slices}, whole 8-slice groups (the forward projector's groups, and whole
-// 4-slice groups of the filter and backprojector, so that a slab-streamed result
-// equals one pass over the whole stack bit for bit; a partial last group goes at
-// the very end). The host->device copy of slab k + 1 and the device->host copy of
-// slab k - 1 run on their own streams while slab k is computed. The schedule
-// tapers at both ends, so the copy in before the first slab and the copy out after
-// the last one, which nothing overlaps, are short. A middle slab holds an eighth
-// of a deep stack (a sixteenth of a shallow one), but enough 32x32 tiles of slice
-// pairs for three per SM, what an SM backprojects at once, and at most a third of
-// the stack; an end slab one tile per SM, at most half a middle one. Measured, ms
-// per call from pinned memory: 256^3 x 360 2.49 (16, 48, 64, 64, 48, 16 slices)
-// against 3.48 in sixteen equal slabs and 3.98 in one; 128^3 x 180 0.55 against
-// 1.26 and 0.64; 512^3 x 720 20.6 (8, 24, 7 x 64, 24, 8; with 128-slice middle slabs
-// 22.0).
-std::vector<int2> plan_slabs(int depth, int n_out, int sms) {
-    std::vector<int2> slabs;
-    if (depth <= 16) {
-        slabs.push_back(make_int2(0, depth));
-        return slabs;
-    }
-    auto groups = [](int slices) { return (slices + 7) / 8 * 8; };  // whole 8-slice groups
-    const int sixteenth = groups((depth + 15) / 16);
-    const int tiles = static_cast<int>(std::min(1LL << 20, (n_out + 31LL) / 32 * ((n_out + 31LL) / 32)));
-    const int fill = 8 * ((3 * sms + tiles - 1) / tiles);
-    const int body = std::min(std::max(fill, sixteenth >= 32 ? 2 * sixteenth : sixteenth), groups((depth + 2) / 3));
-    const int end = std::max(8, std::min(8 * (sms / tiles), body / 16 * 8));
-    const int next = std::min(3 * end, body);
-    const int rem = depth % 8;
-    int left = depth - rem;
-    std::vector<int> taper;
-    for (const int s : {end, next})
-        if (left >= 2 * s + body) {
-            taper.push_back(s);
-            left -= 2 * s;
-        }
-    std::vector<int> sizes = taper;
-    for (int pieces = std::max(1, (left + body / 2) / body); pieces > 0; --pieces) {
-        const int s = std::min(left, groups((left + pieces - 1) / pieces));
-        if (s > 0) sizes.push_back(s);
-        left -= s;
-    }
-    sizes.insert(sizes.end(), taper.rbegin(), taper.rend());
-    if (rem > 0 && sizes.back() + rem <= body) sizes.back() += rem;
-    else if (rem > 0) sizes.push_back(rem);
-    int z = 0;
-    for (const int s : sizes) {
-        slabs.push_back(make_int2(z, s));
-        z += s;
-    }
-    return slabs;
-}
-
 // Host-buffer FBP of a sinogram stack sinos[depth][na][bins] into
 // out[depth][n_out]^2, streamed in slabs (plan_slabs): slab k + 1's sinograms
 // copy in on one stream and slab k - 1's slices copy out on another while slab
@@ -455,14 +402,18 @@ std::vector<int2> plan_slabs(int depth, int n_out, int sms) {
 // time from the first slab's compute to the last one's.
 ctb_status fbp_host_pipeline(ctb_ctx* ctx, const float* sinos, int depth, int na, int bins,
                              const float* angles_deg, int n_out, int filter, int denorm, float* out) {
-    const std::vector<int2> slabs = plan_slabs(depth, n_out, ctx->sms);
-    const int nslab = static_cast<int>(slabs.size());
-    int slab = 0;
-    for (const int2& sl : slabs) slab = std::max(slab, sl.y);
     const size_t row = static_cast<size_t>(na) * bins, img = static_cast<size_t>(n_out) * n_out;
     const PadGeom g = pad_geometry(bins);
     if (g.Lc > kMaxFft)
         return fail(ctx, CTB_ERR_UNSUPPORTED, "convolution length %d (bins %d) exceeds %d", g.Lc, bins, kMaxFft);
+    SlabWork work;
+    work.in = sizeof(float) * row;
+    work.out = sizeof(float) * img;
+    work.scratch = 2 * (work.in + work.out) + sizeof(float) * na * filt_layout(g.sq, n_out).pitch;
+    const std::vector<int2> slabs = plan_slabs(depth, n_out, ctx->sms, work);
+    const int nslab = static_cast<int>(slabs.size());
+    int slab = 0;
+    for (const int2& sl : slabs) slab = std::max(slab, sl.y);
     CTB_WS(ctx, d_sino, float, "h_sino", 2 * static_cast<size_t>(slab) * row);
     CTB_WS(ctx, d_out, float, "h_out", 2 * static_cast<size_t>(slab) * img);
     CTB_WS(ctx, d_stats, float4, "h_stats", 2 * static_cast<size_t>(slab));
@@ -967,7 +918,13 @@ ctb_status ctb_reconstruct_volume(ctb_ctx* ctx, const float* vol, int n, int dep
         num_angles > kMaxAngles)
         return fail(ctx, CTB_ERR_INVALID, "ctb_reconstruct_volume: invalid arguments");
     Guard g(ctx);
-    const std::vector<int2> slabs = plan_slabs(depth, n, ctx->sms);
+    SlabWork work;
+    work.in = work.out = sizeof(float) * static_cast<size_t>(n) * n;
+    work.scratch = 4 * work.in + 2 * sizeof(float) * fwd_plane_elems(n, n) +
+                   sizeof(float) * num_angles *
+                       (2 * static_cast<size_t>(detector_bins) +
+                        filt_layout(pad_geometry(detector_bins).sq, n).pitch);
+    const std::vector<int2> slabs = plan_slabs(depth, n, ctx->sms, work);
     const int nslab = static_cast<int>(slabs.size());
     int slab = 0;  // the largest slab: buffer sizes
     for (const int2& sl : slabs) slab = std::max(slab, sl.y);

@@ -211,6 +211,12 @@ struct FwdPlan {
     int max_strips = 0;
 };
 FwdPlan forward_plan(const float* angles_deg, int na, int w, int h, int nd);
+// Slabs {first slice, slices} of a host-buffer pipeline.
+struct SlabWork {             // of a slice
+    size_t in = 0, out = 0;   // bytes copied to and from the device
+    size_t scratch = 0;       // device bytes of a slab's buffers, all copies of them
+};
+std::vector<int2> plan_slabs(int depth, int n_out, int sms, const SlabWork& work);
 // Per-angle constants of the forward projector, in plan order (slot i holds
 // angle order[i], walked along its group's axis): kq and kp, the coefficients
 // of the gathered and the walked axis, inv = 1 / kq, idq = 1 / dq with
