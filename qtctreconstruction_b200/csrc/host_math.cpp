@@ -288,11 +288,15 @@ FwdPlan forward_plan(const float* angles_deg, int na, int w, int h, int nd) {
 // 0.55 against 1.26 and 0.64; 512^3 x 720 20.6 (8, 24, 7 x 64, 24, 8; with 128-slice
 // middle slabs 22.0).
 //
-// A slab's buffers take no more than kSlabScratch, or what an eighth or sixteenth of
-// the stack takes: with very many angles or bins a third of the stack need not fit the
-// device.
+// Two limits on the middle slab. Its buffers take no more than kSlabScratch beyond
+// what an eighth or sixteenth of the stack takes: with very many angles or bins a
+// third of the stack need not fit the device. And where both copies of an FBP take
+// about as long as each other, and longer than the FBP, a large slab leaves each copy
+// engine idle in turn: it holds about kCopySlab bytes then (us per FBP from pinned
+// memory, 256^2 x 200 x 180 1685 -> 1419 with 16 slices instead of 72, 384^2 x 50 x 180
+// 1000 -> 843 with 8 instead of 32).
 std::vector<int2> plan_slabs(int depth, int n_out, int sms, const SlabWork& work) {
-    constexpr size_t kSlabScratch = size_t(4) << 30;
+    constexpr size_t kSlabScratch = size_t(4) << 30, kCopySlab = 4400000;
     std::vector<int2> slabs;
     if (depth <= 16) {
         slabs.push_back(make_int2(0, depth));
@@ -310,6 +314,10 @@ std::vector<int2> plan_slabs(int depth, int n_out, int sms, const SlabWork& work
         body = std::min(body, std::max(least, whole(kSlabScratch / work.scratch)));
         strict = true;
     }
+    const size_t larger = std::max(work.in, work.out);
+    if (work.copies_lead && 2 * work.in >= work.out && 5 * work.in <= 8 * work.out && 8 * larger >= 1000000)
+        body = std::min(body, whole(kCopySlab / larger));
+    if (work.copies_lead && body * larger > 4000000) strict = true;
     const int end = std::max(8, std::min(8 * (sms / tiles), body / 16 * 8));
     const int next = std::min(3 * end, body);
     const int rem = depth % 8;

@@ -2,7 +2,8 @@
 
 plan_slabs (csrc/host_math.cpp) over random stacks: whole groups of 8 slices in
 order, nothing left out; slabs whose buffers would take more than 4 GiB hold no more
-than an eighth or a sixteenth of the stack.
+than an eighth or a sixteenth of the stack; and where an FBP is bound by copies that
+take alike both ways, a slab is a few megabytes.
 """
 import os
 import random
@@ -23,6 +24,7 @@ int main() {
     int depth, n, sms, lead;
     ctb::SlabWork w;
     while (std::scanf("%d %d %d %zu %zu %zu %d", &depth, &n, &sms, &w.in, &w.out, &w.scratch, &lead) == 7) {
+        w.copies_lead = lead;
         for (const int2& s : ctb::plan_slabs(depth, n, sms, w)) std::printf("%d,%d ", s.x, s.y);
         std::printf("\n");
     }
@@ -69,3 +71,6 @@ def test_schedule(tmp_path):
         most = max(c for _, c in slabs)
         # a piece is at most half a slab larger than the middle slab it is one of
         assert most * scratch <= max(1.5 * 4 * 2 ** 30, (_least(depth) + 7) * scratch), (depth, n, scratch, slabs)
+        larger = max(size_in, out)
+        if lead and 2 * size_in >= out and 5 * size_in <= 8 * out and 8 * larger >= 1000000:
+            assert most <= max(8, 4400000 // larger) + 7, (depth, n, size_in, out, slabs)
