@@ -240,8 +240,10 @@ FwdPlan forward_plan(const float* angles_deg, int na, int w, int h, int nd) {
     std::vector<int> lists[2];
     std::vector<double> akq(na), slope(na);
     for (int a = 0; a < na; ++a) {
-        // the projector's own trig (k_trig): sincospi of deg / 180 in double
-        const double t = static_cast<double>(angles_deg[a]) / 180.0;
+        // the projector's own trig (k_trig): sincospi of deg / 180 in double; whole
+        // turns leave first (exactly), or pi t loses the direction of angles from
+        // about 1e16 degrees on, and a walk along the wrong axis leaves the planes
+        const double t = std::fmod(static_cast<double>(angles_deg[a]) / 180.0, 2.0);
         const double cs = std::cos(3.14159265358979323846 * t), sn = std::sin(3.14159265358979323846 * t);
         const double c = std::fabs(cs), s = std::fabs(sn);
         const int axis = c >= s ? 0 : 1;
