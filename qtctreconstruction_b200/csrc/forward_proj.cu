@@ -84,13 +84,16 @@ struct FAngle {
 };
 
 __device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
-// One pixel of a plane pair: 8 slices in 32 bytes (32-byte aligned), one load
-// (ld_chained: the normalisation before this kernel may still run when it starts).
+// One pixel of a plane pair: 8 slices in 32 bytes (32-byte aligned), one load, not
+// through the read-only path (the normalisation before this kernel may still run when
+// it starts). It stays behind chain_wait without being volatile, because its address
+// comes from a row record written after the block's barrier; volatile keeps the loads
+// from being spread over a row group's arithmetic (1148 -> 1165 us at 387^2 x 50 x 580).
 __device__ __forceinline__ void ld_pixel(const float4* p, float4 (&v)[NP]) {
-    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[0].z), "=f"(v[0].w), "=f"(v[1].x), "=f"(v[1].y),
-                   "=f"(v[1].z), "=f"(v[1].w)
-                 : "l"(p));
+    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[0].z), "=f"(v[0].w), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[1].z),
+          "=f"(v[1].w)
+        : "l"(p));
 }
 __device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
 
