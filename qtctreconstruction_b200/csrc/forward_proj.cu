@@ -239,7 +239,8 @@ __device__ __noinline__ float edge_bin(const float* plane, int pitch, int nq, co
 // loads: four per SM (127 registers) let a warp have all eight rows of a group on
 // their way (us of a whole call, seven against four: 45.1 and 33.4 at 160^2 x 1 x
 // 180, 39.0 and 29.8 at 128^2 x 8 x 180, 28.7 and 22.6 at 64^2 x 1 x 90; but 72.0
-// and 73.3 at 256^2 x 1 x 360 with 1620 CTAs, 2563 and 2714 at 512^2 x 64 x 720).
+// and 73.3 at 256^2 x 1 x 360 with 1620 CTAs, 2563 and 2714 at 512^2 x 64 x 720). A
+// single slice in planes of its own needs 72 registers either way.
 constexpr int FULL = 7, SPARSE = 4;
 // ONE: a single slice in planes of 4-byte pixels (img, imgT then point to floats):
 // a row of 32 columns is one or two L1 wavefronts instead of nine and a row takes a
@@ -559,8 +560,7 @@ cudaError_t launch_forward(const float4* d_img, const float4* d_imgT, int w, int
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const bool sparse = static_cast<long long>(grid.x) * grid.y * grid.z <= static_cast<long long>(SPARSE) * sms;
-    auto kernel = single ? (sparse ? k_forward<SPARSE, true> : k_forward<FULL, true>)
-                         : (sparse ? k_forward<SPARSE, false> : k_forward<FULL, false>);
+    auto kernel = single ? k_forward<FULL, true> : sparse ? k_forward<SPARSE, false> : k_forward<FULL, false>;
     return launch_chained(kernel, grid, dim3(LANES, GMAX), 0, st, d_img, d_imgT, w,
                           h, nz, na, nd, d_groups, d_rec, d_box, d_band, d_sino);
 }
