@@ -56,6 +56,17 @@ inline T* ws(ctb_ctx* ctx, const char* name, size_t count) {
     if (!var) return fail((ctx), CTB_ERR_OOM, "device workspace '%s' (%zu bytes) failed", \
                           (name), static_cast<size_t>(count) * sizeof(T))
 
+// A host buffer the copy engines can read or write directly (page-locked by
+// cudaHostAlloc or cudaHostRegister).
+inline bool page_locked(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost;
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Float degrees 180/na * a (SerialBackend.cpp:126-130).

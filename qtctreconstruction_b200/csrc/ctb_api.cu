@@ -410,7 +410,7 @@ ctb_status fbp_host_pipeline(ctb_ctx* ctx, const float* sinos, int depth, int na
     work.in = sizeof(float) * row;
     work.out = sizeof(float) * img;
     work.scratch = 2 * (work.in + work.out) + sizeof(float) * na * filt_layout(g.sq, n_out).pitch;
-    work.copies_lead = true;
+    work.copies_lead = page_locked(sinos) && page_locked(out);  // others hold up the calling thread
     const std::vector<int2> slabs = plan_slabs(depth, n_out, ctx->sms, work);
     const int nslab = static_cast<int>(slabs.size());
     int slab = 0;

@@ -215,7 +215,7 @@ FwdPlan forward_plan(const float* angles_deg, int na, int w, int h, int nd);
 struct SlabWork {             // of a slice
     size_t in = 0, out = 0;   // bytes copied to and from the device
     size_t scratch = 0;       // device bytes of a slab's buffers, all copies of them
-    bool copies_lead = false; // FBP alone: of few hundred angles it is faster than its copies
+    bool copies_lead = false; // FBP alone, page-locked: its copies overlap, and may take longer
 };
 std::vector<int2> plan_slabs(int depth, int n_out, int sms, const SlabWork& work);
 // Per-angle constants of the forward projector, in plan order (slot i holds

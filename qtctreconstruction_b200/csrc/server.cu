@@ -495,18 +495,6 @@ bool upload_trig(SReq* q, Stager& st) {
            cudaStreamSynchronize(st.stream) == cudaSuccess;
 }
 
-// A host buffer the copy engines can read or write directly (page-locked by
-// cudaHostAlloc or cudaHostRegister); pageable memory goes through the pinned
-// double buffers.
-bool page_locked(const void* p) {
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return a.type == cudaMemoryTypeHost;
-}
-
 // Host -> device: straight from page-locked memory, else through the pinned
 // double buffer (chunk k is copied into buffer k & 1 once that buffer's
 // previous transfer has finished).
