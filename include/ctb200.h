@@ -118,17 +118,20 @@ ctb_status ctb_filter_kernel_ms(ctb_ctx* ctx, int back, double* ms);
 enum { CTB_FILTER_MODE_FFT = 0, CTB_FILTER_MODE_TC_BF16X3 = 1 };
 ctb_status ctb_set_filter_mode(ctb_ctx* ctx, int mode);
 
-/* Backprojection tile shapes. Six are compiled: 0 = 32x32 voxels, 4 per
- * thread (the general case); 1 = 64x32, 8 per thread; 2 = 32x16, 2 per
- * thread; 3 = 16x16, 1 per thread; all with 32 angles per staged chunk; and
- * the 32x32 tile with 16 (4) and 64 (5) angles per chunk, which sum every
- * voxel's angles in the same order as shape 0 and so give its result bit for
- * bit. (A chunk is half the ring of staged windows, one window per angle and
- * group of four slices.) Without tuning a job gets a shape from its size alone:
+/* Backprojection tile shapes. Six are compiled: 0 = 32x32 voxels (the general
+ * case), 1 = 64x32, 2 = 32x16, 3 = 16x16, and the 32x32 tile with half (4) and
+ * twice (5) the ring of staged windows, which sum every voxel's angles in the same
+ * order as shape 0 and so give its result bit for bit. A thread owns columns of four
+ * voxels; small tiles split the angles over groups of threads. A stage holds 26, 16,
+ * 24, 24, 12 and 32 windows (shapes 0 to 5), one per angle and group of four slices,
+ * and a ring 3, 4, 4, 4, 3 and 4 stages. ctb_bp_shape_info reports the tile's edges,
+ * its voxels over the CTA's 256 threads, and a nominal number of angles (32; 16 and
+ * 64 for shapes 4 and 5) that the stages do not follow.
+ * Without tuning a job gets a shape from its size alone:
  * 32x32, or 32x16 or 16x16 where its tiles would leave SMs idle; jobs of few angles
  * (24, or up to 64 where their tiles leave SMs idle) take such a tile in a kernel of
  * their own, which is neither tuned nor forced. With the autotuner
- * on, the first job of each size bucket {ceil(n / 64), ceil(angles / 180),
+ * on, the first other job of each size bucket {ceil(n / 64), ceil(angles / 180),
  * floor(log2(ceil(depth / 4)))} times every shape on its own data (that call
  * synchronises) and the fastest is kept for the bucket; batches use a tuned
  * shape when their job's bucket is tuned, else the default, so a job's shape

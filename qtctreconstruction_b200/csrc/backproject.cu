@@ -36,7 +36,7 @@
 // the slow coefficient alone (four patterns, column_taps), and two slice groups
 // share the weights. The kernel is then bound by issue: 44 packed FP32x2 FMAs of
 // two issue cycles (6.2 ms on their own) and about 43 other instructions per column
-// and angle of 8 slices: 10.46 ms at 512^3 x 720, FMA pipe 69 %, shared memory 78 %
+// and angle of 8 slices: 10.57 ms at 512^3 x 720, FMA pipe 69 %, shared memory 78 %
 // busy (11.03 ms with smaller stages, see Shape). Measured then, against 11.03: with
 // two of the taps read only, 10.95 ms; not kept: tap differences with saturating
 // weights, which share the first tap's sum within a column (11.72), one slice group
@@ -74,7 +74,8 @@ constexpr float kRound = 12582912.0f;   // 1.5 * 2^23: x + kRound rounds x to an
 constexpr int kRoundBits = 0x4B400000;  // bit pattern of kRound
 
 // A tile shape: TX x TY voxels in columns of V, a ring of NST stages of SW windows
-// (one per angle and slice group; about 2 CA in all) and WIN bins per window: with
+// (one per angle and slice group; CA is a nominal count that bp_shape reports, the
+// stages do not follow it) and WIN bins per window: with
 // a span of sqrt((TX-1)^2 + (TY-1)^2) bins, the taps of every column lie in bins 0
 // .. floor(span + 2) + 2 of the window. MINB is the launch-bounds occupancy target
 // (registers 65536 / (256 MINB)). A stage costs every warp about 80 instructions
@@ -110,8 +111,8 @@ using V3 = Shape<16, 16, 32, 28, 24, 4, 3, true>;  // small tiles for small slic
 using V4 = Shape<32, 32, 16, 48, 12, 3, 3, true>;  // the general shape with half the ring
 using V5 = Shape<32, 32, 64, 48, 32, 4, 2, true>;  // the general shape with twice the ring (half the stages)
 
-// A tile shape of jobs with few angles (few_tile): TX x TY voxels of four slices, VPT voxels per thread along x (TX / VPT apart), 32 angles per staged
-// chunk.
+// A tile shape of jobs with few angles (few_tile): TX x TY voxels of four slices, VPT
+// voxels per thread along x (TX / VPT apart), 32 angles per staged chunk.
 template <int TX_, int TY_, int VPT_, int WIN_>
 struct Few {
     static constexpr int TX = TX_, TY = TY_, VPT = VPT_, CA = 32, WIN = WIN_, MINB = 4;
@@ -677,8 +678,9 @@ template <> struct FewOf<V0> : FewIn<F0, V0> {};
 template <> struct FewOf<V2> : FewIn<F2, V2> {};
 template <> struct FewOf<V3> : FewIn<F3, V3> {};
 
-// Backproject one tile (x0, y0) of slice group zg of job J. bar: one per buffer. `chunks` counts the
-// chunks this CTA has consumed so far (mbarrier phases continue across items).
+// Backproject one tile (x0, y0) of slice group zg of job J. bar: one per buffer.
+// `chunks` counts the chunks this CTA has consumed so far (mbarrier phases continue
+// across items).
 // Returns false when a bounded wait gave up (block-uniform), the copies under way
 // waited for.
 template <class C>
@@ -1089,8 +1091,10 @@ long long active_tiles(int n, const BpShape& sh, double ctr) {
 // the fullest SM decides, a lone item taking 1.4 times its share of a full SM
 // (its 8 warps do not fill it); beyond it the SMs even out to half an item.
 // Costs per item (one or two slice groups) relative to a 32x32 tile of one group,
-// from the backprojector's time at 512^2 x 64 x 720 (with stages of 16 windows):
-// 32x32 1.658 and 1.462 ms, 32x16 1.822 and 1.640, 16x16 2.173 and 2.082.
+// from the backprojector's time at 512^2 x 64 x 720 with stages of 16 windows: 32x32
+// 1.658 and 1.462 ms, 32x16 1.822 and 1.640, 16x16 2.173 and 2.082. With the present
+// stages an FBP takes 1.792 and 1.581, 1.933 and 1.714, 2.281 and 2.063 (0.18 of it
+// the filter): 1.73 for a pair, 0.54 and 0.95, 0.33 and 0.58.
 double launch_cost(int variant, int zgs, long long items, int sms) {
     const double pair = variant == 2 ? 0.99 : variant == 3 ? 0.63 : 1.76;
     const double one = variant == 2 ? 0.55 : variant == 3 ? 0.33 : 1.0;
@@ -1143,7 +1147,7 @@ int bp_default_variant(int n_out, int nz, int na, int sms) {
 }
 
 void bp_number_items(BpBatch& b, int variant, int sms) {
-    // Pairs of slice groups share every weight (1.46 against 1.66 ms at 512^2 x
+    // Pairs of slice groups share every weight (FBP 1.58 against 1.79 ms at 512^2 x
     // 64 x 720) but make half as many items, which costs more than it gives
     // where the items do not fill the SMs (58.8 against 40.4 us at 128^2 x 32
     // x 201). A slice's result does not depend on the choice.

@@ -4,9 +4,10 @@
 // The reference reconstructs one volume per call (IReconstructionBackend.h:
 // 39-44); a batch takes a list of (sinogram stack, geometry, filter) jobs and
 // runs the filter stage of all jobs that share a convolution length in one
-// launch and the backprojection of all jobs in one persistent launch whose
-// work queue holds (job, slice group, tile) items, the jobs with the most
-// angles first so that the cheap items fill the tail. Items never share an
+// launch and the backprojection of all jobs that share a tile shape in another,
+// one CTA per (job, slice groups, tile) item (CTB_BATCH_PERSISTENT: a resident
+// grid drawing the items from a counter), the jobs with the most angles first so
+// that the cheap items fill the tail. Items never share an
 // output value, so each job's result is bit-identical to ctb_fbp_d on that job
 // alone. With CTB_BATCH_GRAPH the launches are captured once into a CUDA graph
 // and each run replays it.

@@ -76,6 +76,30 @@ def test_denormalised_volume_meets_parity(backend):
     assert O.rel_l2(d_o.cpu().numpy(), ref) <= 1e-5
 
 
+@pytest.mark.parametrize("convention", [ctb.CONVENTION_SERIAL, ctb.CONVENTION_CUDA])
+@pytest.mark.parametrize("n,bins,na", [(64, 91, 20), (90, 40, 33)])
+def test_conventions_equal_the_columns(backend, convention, n, bins, na):
+    """Both conventions' grids and tap rules, against the columns (shape 3)."""
+    import torch
+    sinos = torch.from_numpy(np.random.default_rng(na).uniform(0.0, 1.0, (5, na, bins)).astype(np.float32)).cuda()
+    outs = []
+    backend.set_convention(convention)
+    try:
+        for shape in (-1, 3):
+            backend.set_bp_shape(shape)
+            o = torch.full((5, n, n), float("nan"), device="cuda")
+            torch.cuda.synchronize()
+            backend.fbp_d(sinos.data_ptr(), 5, na, bins, n, int(FilterType.Hann), o.data_ptr())
+            backend.synchronize()
+            outs.append(o.cpu().numpy())
+    finally:
+        backend.set_bp_shape(-1)
+        backend.set_convention(ctb.CONVENTION_SERIAL)
+    assert np.all(np.isfinite(outs[0]))
+    assert O.rel_l2(outs[0], outs[1]) <= 1e-5
+    assert O.max_abs_rel(outs[0], outs[1]) <= 1e-4
+
+
 def test_few_angles_are_not_slower_than_the_columns(backend):
     """8 angles over 512^2 x 4 are 8 of the columns' groups: 15 us a call in columns, 12
     without. The automatic choice, timed in turn with the forced shapes, is at least a
