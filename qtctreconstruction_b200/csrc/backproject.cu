@@ -230,7 +230,7 @@ struct BpSmem {
     float2 ex[C::SPLIT * C::TX * C::TY];     // exchange of accumulators between threads
     AngleRec rec[NST][C::SW + C::SPLIT];     // a record is read ahead of its use
     unsigned long long full[NST], empty[NST];
-    int meta[NST];                           // stage: angles | some angle has `edge` set << 8
+    int meta[NST];                           // stage: angles | group << 8 | some angle has `edge` set << 16
     unsigned sent[NST];                      // stages whose copies were issued into the slot
     int first[kBpGroups];                    // first stage of each group of the angle order
     int start[kBpGroups + 1];                // first angle of each group; na
@@ -363,9 +363,6 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
     }
     __syncthreads();
     const int total = S.total;
-    // the group of a stage: the last one that starts at or before it
-    const int my_first = lane < kBpGroups ? S.first[lane] : INT_MAX;
-    auto group_of = [&](int i) { return __popc(__ballot_sync(0xffffffffu, my_first <= i)) - 1; };
     auto wait = [&](unsigned long long* bar, unsigned parity) {
         const bool ok = mbar_wait_bounded(bar, parity, err, LOST ? lost.limit_ns : kWaitLimitNs, 1u, &S.dead);
         if (!ok) *static_cast<volatile int*>(&S.dead) = 1;
@@ -381,7 +378,8 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
         bool ok = *static_cast<volatile int*>(&S.dead) == 0;
         if (ok && use > 0) ok = wait(&S.empty[slot], (use - 1) & 1);
         if (!__all_sync(0xffffffffu, ok)) return;  // nothing is copied any more
-        const int grp = group_of(i);
+        // the last group that starts at or before stage i
+        const int grp = __popc(__ballot_sync(0xffffffffu, lane < kBpGroups && S.first[lane & (kBpGroups - 1)] <= i)) - 1;
         const int pos = S.start[grp] + (i - S.first[grp]) * SA;
         const int cnt = min(SA, S.start[grp + 1] - pos);
         const bool along = grp < kBpGroups / 2, flip = (grp / 4) & 1;
@@ -415,7 +413,7 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
         edge = __any_sync(0xffffffffu, edge);
         const bool send = !LOST || i != lost.stage;
         if (lane == 0) {
-            S.meta[slot] = cnt | (edge ? 1 << 8 : 0);
+            S.meta[slot] = cnt | grp << 8 | (edge ? 1 << 16 : 0);
             if (send) S.sent[slot] = use + 1;
         }
         __syncwarp();
@@ -521,7 +519,15 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
         // A failed wait leaves stale records and windows: the warp takes nothing of
         // them, and the block stops as a whole at the end of the item.
         landed = landed && wait(&S.full[slot], (stages / NST) & 1);
-        const int grp = group_of(i);
+        // cnt | grp << 8 of the stage; without the stage its group alone, so that every
+        // warp passes the block's barriers in exchange() at the same stage
+        int meta = 0;
+        if (landed) {
+            meta = S.meta[slot];
+        } else {
+            for (int q = 1; q < kBpGroups; ++q) meta += S.first[q] <= i ? 1 << 8 : 0;
+        }
+        const int cnt = meta & 0xff, grp = (meta >> 8) & 0xff;
         if (along_x && grp >= kBpGroups / 2) exchange();
         if (flipped != (((grp / 4) & 1) != 0)) flip_columns();
         const float fi = static_cast<float>(fast);
@@ -532,7 +538,6 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
             fj[k] = static_cast<float>(V * col[k]);
             some |= live[k];
         }
-        const int meta = landed ? S.meta[slot] : 0, cnt = meta & 0xff;
         if (some && g < cnt) {
             // 32-bit shared addresses of this group's first record and window;
             // the window's is offset so that adding 16 times the bits of
@@ -591,7 +596,7 @@ __device__ __forceinline__ bool bp_tile(BpSmem<C>& S, const BpJob& J, int zg, in
                 else if (pat == 2) run(std::integral_constant<int, 2>(), edges);
                 else run(std::integral_constant<int, 3>(), edges);
             };
-            if (meta >> 8) run_pattern(std::true_type());
+            if (meta >> 16) run_pattern(std::true_type());
             else run_pattern(std::false_type());
         }
         __syncwarp();
