@@ -36,7 +36,7 @@
 // the slow coefficient alone (four patterns, column_taps), and two slice groups
 // share the weights. The kernel is then bound by issue: 44 packed FP32x2 FMAs of
 // two issue cycles (6.2 ms on their own) and about 43 other instructions per column
-// and angle of 8 slices: 10.57 ms at 512^3 x 720, FMA pipe 69 %, shared memory 78 %
+// and angle of 8 slices: 10.55 ms at 512^3 x 720, FMA pipe 69 %, shared memory 78 %
 // busy (11.03 ms with smaller stages, see Shape). Measured then, against 11.03: with
 // two of the taps read only, 10.95 ms; not kept: tap differences with saturating
 // weights, which share the first tap's sum within a column (11.72), one slice group
